@@ -18,9 +18,8 @@
 namespace vpm {
 
 constexpr int kMaxLevels3D = 60;     // octree depth limit (coincident particles)
-constexpr int kWork3DCap = 512;      // union work list of a warp's traversal per level, at support
-                                     // factor 2 (eval3d scales it for larger factors)
-constexpr int kEval3DWarps = 4;      // warps (leaves) per evaluation block
+constexpr int kMom3D = 30;           // doubles per cell's moments
+constexpr int kRec32Floats = 36;     // mixed form: 3 doubles (centre) and 30 floats per cell
 constexpr int kCoopMaxBlocks3D = 148 * 8;  // size of the per-block scan partials
 
 // Geometry record of the bounding-box kernel (fast3DFMM.cpp:485-520 with the
@@ -68,11 +67,12 @@ struct Tree3D {
     int32_t *c_npar, *c_parent, *c_child0, *c_lo, *c_hi;
     uint32_t* c_chmask;               // child octants present (reference chdFlag)
     uint8_t *c_active, *c_level;
-    double* mom;                      // [cap_cells][30]: moments of alpha_x, alpha_y, alpha_z
-    // mixed form: FP32 copies made once per evaluation (prep3d_f32)
+    double* mom;                      // [cap_cells][kMom3D]: moments of alpha_x, alpha_y, alpha_z, then
+                                      // (prep3d, plain form) the evaluation's record
+    // mixed form: FP32 copies made once per evaluation (prep3d)
     float4* ps32;                     // position minus its leaf's centre, active flag in .w
     float4* as32;                     // alpha
-    float* mom32;                     // [cap_cells][30]
+    float* rec32;                     // [cap_cells][kRec32Floats]: centre (doubles), moments
     int32_t* leaf_cells;              // leaves in cell order
     unsigned* gbar;                   // grid barrier words (2), zeroed per evaluation
     uint32_t* blk;                    // per-block scan partials [gridDim]
@@ -107,10 +107,11 @@ cudaError_t build_treecell3d(const double* x, const double* y, const double* z, 
                              double exp_pct, Tree3D& t, Scratch3D& s, double* bbox_partial, unsigned* err,
                              cudaStream_t st, int* launches);
 
-// FP32 copies for the mixed traversal: each particle's offset from its
-// leaf's centre (formed in FP64, rounded once) with its active flag, its
-// alpha, and every cell's moments.
-cudaError_t prep3d_f32(const Tree3D& t, unsigned* err, cudaStream_t st, int* launches);
+// What the evaluation reads, made once after M2M. Mixed form: FP32 copies of
+// each particle's offset from its leaf's centre (formed in FP64, rounded
+// once) with its active flag, its alpha, and every cell's moments. Plain
+// form: every cell's moments rewritten in place as the FP64 M2P's record.
+cudaError_t prep3d(const Tree3D& t, bool mixed, unsigned* err, cudaStream_t st, int* launches);
 
 // Per-target traversal (M2P of far cells, P2P of near leaves) writing the
 // velocity u = sum alpha x r / |r|^3 (+ free stream) in the caller's order.

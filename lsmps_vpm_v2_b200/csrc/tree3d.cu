@@ -380,7 +380,7 @@ p2m3d(Tree3D t, unsigned* err) {
                 p2m_term(m, j, src[s], xc - t.px[s], yc - t.py[s], zc - t.pz[s]);
             }
         }
-        if (lane < 30) t.mom[(size_t)c * 30 + lane] = m;
+        if (lane < 30) t.mom[(size_t)c * kMom3D + lane] = m;
     }
 }
 
@@ -403,7 +403,7 @@ __device__ __forceinline__ void m2m3d_level(const Tree3D& t, int L) {
             if (!((mask >> o) & 1u)) continue;
             const int k = k0 + r++;
             const double dx = xc - t.c_x[k], dy = yc - t.c_y[k], dz = zc - t.c_z[k];
-            const double* ch = &t.mom[(size_t)k * 30 + 10 * a];
+            const double* ch = &t.mom[(size_t)k * kMom3D + 10 * a];
             const double c_0 = __ldcg(&ch[0]), c_1 = __ldcg(&ch[1]), c_2 = __ldcg(&ch[2]), c_3 = __ldcg(&ch[3]);
             const double cj = __ldcg(&ch[j]);
             switch (j) {
@@ -419,7 +419,7 @@ __device__ __forceinline__ void m2m3d_level(const Tree3D& t, int L) {
                 default: m += cj + (c_0 * dx * dz) + (c_1 * dz) + (c_3 * dx); break;
             }
         }
-        t.mom[(size_t)c * 30 + lane] = m;
+        t.mom[(size_t)c * kMom3D + lane] = m;
     }
 }
 
