@@ -35,6 +35,7 @@ struct Geom3D {
 // iz 4^L are 32-bit ints in the reference (treeCell.cpp:223-250) and overflow
 // from level 11 on. Keys hold 3 bits per level.
 constexpr int kTcLevels = 10;
+constexpr int kDeepWord = 5;    // word of Tree3D::gbar: an octree cell of level kTcLevels has to be split
 constexpr int kTcTile = 1024;   // particles per tile of the level-count scan
 
 struct TreeInfo3D {
@@ -74,7 +75,7 @@ struct Tree3D {
     float4* as32;                     // alpha
     float* rec32;                     // [cap_cells][kRec32Floats]: centre (doubles), moments
     int32_t* leaf_cells;              // leaves in cell order
-    unsigned* gbar;                   // grid barrier words (2), zeroed per evaluation
+    unsigned* gbar;                   // grid barrier words, the octree's kDeepWord; zeroed per evaluation
     uint32_t* blk;                    // per-block scan partials [gridDim]
 };
 

@@ -104,35 +104,28 @@ bbox3d(const double* __restrict__ x, const double* __restrict__ y, const double*
     }
 }
 
-// Root cell and the per-particle build state (fast3DFMM.cpp:533-550, 620-625).
-__global__ void root3d(Tree3D t) {
-    const int n = t.n;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        t.pcell[i] = 0;
-        t.settled[i] = 0;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        const Geom3D* g = t.geom;
-        t.c_x[0] = g->cen[0];
-        t.c_y[0] = g->cen[1];
-        t.c_z[0] = g->cen[2];
-        t.c_size[0] = g->root;
-        t.c_npar[0] = n;
-        t.c_parent[0] = -1;
-        t.c_child0[0] = -1;
-        t.c_chmask[0] = 0;
-        t.c_active[0] = 1;
-        t.c_level[0] = 0;
-        TreeInfo3D* info = t.info;
-        for (int L = 0; L < kMaxLevels3D + 2; ++L) info->level_start[L] = L == 0 ? 0 : 1;
-        info->n_cells = 1;
-        info->n_leaves = 0;
-        info->depth = 0;
-        info->remaining = n;
-        info->scan_total = 0;
-        info->p2p_pairs = 0;
-        info->m2p_pairs = 0;
-    }
+// Root cell (fast3DFMM.cpp:533-550): level starts and the record of cell 0.
+__device__ __forceinline__ void octree_root(const Tree3D& t) {
+    const Geom3D* g = t.geom;
+    t.c_x[0] = g->cen[0];
+    t.c_y[0] = g->cen[1];
+    t.c_z[0] = g->cen[2];
+    t.c_size[0] = g->root;
+    t.c_npar[0] = t.n;
+    t.c_parent[0] = -1;
+    t.c_child0[0] = -1;
+    t.c_chmask[0] = 0;
+    t.c_active[0] = 1;
+    t.c_level[0] = 0;
+    TreeInfo3D* info = t.info;
+    for (int L = 0; L < kMaxLevels3D + 2; ++L) info->level_start[L] = L == 0 ? 0 : 1;
+    info->n_cells = 1;
+    info->n_leaves = 0;
+    info->depth = 0;
+    info->remaining = t.n;
+    info->scan_total = 0;
+    info->p2p_pairs = 0;
+    info->m2p_pairs = 0;
 }
 
 __device__ __forceinline__ int block_sum_int(int v, int* s_red) {
@@ -177,10 +170,22 @@ __device__ __forceinline__ int block_excl_int(int v, int* s_warp, int* total) {
 // ancestors active when the particle is active (equivalent to the reference's
 // bottom-up pass, fast3DFMM.cpp:711-741). Grid barriers separate the steps;
 // data written by other blocks is read through L2. A particle is always
-// handled by the same thread, so its own state needs no barrier.
+// handled by the same thread, so its own state needs no barrier. Flags and
+// counts are combined per warp first: neighbours in the caller's order mostly
+// share a cell, and two million particles on the root's one word took 8.3 ms.
+//
+// The builds with small leaves use the flat construction below instead (0.15
+// and 0.42 ms up to the leaf ranges on the 222,688- and 2,009,183-particle
+// rings, where this kernel alone took 1.0 and 8.3 before flags and counts
+// were combined, and takes five grid barriers per level at any size) and
+// come here (PLACE) only when a cell at its deepest level still has to be
+// split, told by gbar word kDeepWord; the kernel then also writes the leaf
+// ranges and the particles of each leaf into `order` (in any order: they are
+// sorted by index where the leaf is gathered).
+template <bool PLACE>
 __global__ void __launch_bounds__(kT3Threads)
 octree_levels3d(Tree3D t, const double* __restrict__ x, const double* __restrict__ y,
-                const double* __restrict__ z, const uint8_t* __restrict__ act, int max_blocks, unsigned* err) {
+                const double* __restrict__ z, const uint8_t* __restrict__ act, uint32_t* __restrict__ order, int max_blocks, unsigned* err) {
     __shared__ int s_red[kT3Threads / 32];
     __shared__ int s_warp[kT3Threads / 32];
     __shared__ int s_carry;
@@ -188,9 +193,16 @@ octree_levels3d(Tree3D t, const double* __restrict__ x, const double* __restrict
         if (blockIdx.x == 0 && threadIdx.x == 0) set_err(err, ERR_INDEX);
         return;  // uniform: every block sees the same gridDim
     }
+    if (PLACE && __ldcg(t.gbar + kDeepWord) == 0) return;   // uniform: set by an earlier kernel only
     TreeInfo3D* info = t.info;
     const int n = t.n, cap = t.leaf_cap;
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gstride = gridDim.x * blockDim.x;
+    for (int i = gtid; i < n; i += gstride) {
+        t.pcell[i] = 0;
+        t.settled[i] = 0;
+    }
+    if (gtid == 0) octree_root(t);
+    grid_sync(t.gbar, err);
     for (int L = 1; L <= kMaxLevels3D; ++L) {
         if (__ldcg(&info->remaining) <= 0) break;  // written before the last barrier: uniform
         const bool skip = block_fatal(err);  // per block; barriers are still taken by everyone
@@ -203,7 +215,9 @@ octree_levels3d(Tree3D t, const double* __restrict__ x, const double* __restrict
                 const int oct = (x[i] > __ldcg(&t.c_x[c])) * 1 + (y[i] > __ldcg(&t.c_y[c])) * 2 +
                                 (z[i] > __ldcg(&t.c_z[c])) * 4;
                 t.poct[i] = (uint8_t)oct;
-                atomicOr(&t.c_chmask[c], 1u << oct);
+                const unsigned peers = __match_any_sync(__activemask(), (unsigned)c * 8u + (unsigned)oct);
+                if ((threadIdx.x & 31) == __ffs(peers) - 1 && !((__ldcg(&t.c_chmask[c]) >> oct) & 1u))
+                    atomicOr(&t.c_chmask[c], 1u << oct);
             }
         }
         grid_sync(t.gbar, err);
@@ -281,7 +295,8 @@ octree_levels3d(Tree3D t, const double* __restrict__ x, const double* __restrict
                     continue;
                 }
                 t.pcell[i] = k;
-                atomicAdd(&t.c_npar[k], 1);
+                const unsigned peers = __match_any_sync(__activemask(), k);
+                if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&t.c_npar[k], __popc(peers));
             }
         }
         grid_sync(t.gbar, err);
@@ -306,6 +321,44 @@ octree_levels3d(Tree3D t, const double* __restrict__ x, const double* __restrict
         grid_sync(t.gbar, err);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0 && __ldcg(&info->remaining) > 0) set_err(err, ERR_DEPTH);
+    if (!PLACE) return;
+    grid_sync(t.gbar, err);
+    // leaf ranges: block b owns a contiguous chunk of cells
+    const bool skip = block_fatal(err);
+    const int nc = skip ? 0 : __ldcg(&info->n_cells);
+    const int per = ceil_div(nc, (int)gridDim.x);
+    const int b0 = min(nc, (int)blockIdx.x * per), b1 = min(nc, ((int)blockIdx.x + 1) * per);
+    auto held = [&](int c) { return c > 0 && __ldcg(&t.c_chmask[c]) == 0 ? __ldcg(&t.c_npar[c]) : 0; };
+    int mine = 0, leaves = 0;
+    for (int c = b0 + threadIdx.x; c < b1; c += blockDim.x) {
+        const int v = held(c);
+        mine += v;
+        leaves += v > 0;
+    }
+    mine = block_sum_int(mine, s_red);
+    leaves = block_sum_int(leaves, s_red);
+    if (threadIdx.x == 0) {
+        t.blk[blockIdx.x] = (uint32_t)mine;
+        if (leaves) atomicAdd(&info->n_leaves, leaves);
+    }
+    grid_sync(t.gbar, err);
+    int base = 0;
+    for (int b = threadIdx.x; b < (int)blockIdx.x; b += blockDim.x) base += (int)__ldcg(&t.blk[b]);
+    base = block_sum_int(base, s_red);
+    for (int c0 = b0; c0 < b1; c0 += blockDim.x) {
+        const int c = c0 + threadIdx.x;
+        int tot;
+        const int at = base + block_excl_int(c < b1 ? held(c) : 0, s_warp, &tot);
+        if (c < b1) t.c_lo[c] = t.c_hi[c] = at;   // c_hi: the leaf's cursor below
+        base += tot;
+    }
+    grid_sync(t.gbar, err);
+    if (skip) return;
+    for (int i = gtid; i < n; i += gstride) {
+        const int at = atomicAdd(&t.c_hi[t.pcell[i]], 1);
+        if (at < n) order[at] = (uint32_t)i;
+        else set_err(err, ERR_INDEX);
+    }
 }
 
 // Leaf ranges after the particles were sorted by leaf: key[j] = leaf of the
@@ -343,21 +396,15 @@ __global__ void leaf_keys3d(Tree3D t, uint32_t* key, uint32_t* idx) {
     }
 }
 
-__device__ __forceinline__ void p2m_term(double& m, int j, double s, double dx, double dy, double dz) {
-    // fmm3D.cpp:84-103, one of the ten moments
-    switch (j) {
-        case 0: m += s; break;
-        case 1: m += s * dx; break;
-        case 2: m += s * dy; break;
-        case 3: m += s * dz; break;
-        case 4: m += s * dx * dx * 0.5; break;
-        case 5: m += s * dy * dy * 0.5; break;
-        case 6: m += s * dz * dz * 0.5; break;
-        case 7: m += s * dx * dy; break;
-        case 8: m += s * dy * dz; break;
-        default: m += s * dx * dz; break;
-    }
-}
+// One of the ten moments about a cell's centre (fmm3D.cpp:84-103): 1, x, y, z,
+// xx / 2, yy / 2, zz / 2, xy, yz, xz, as s f1 f2 f3 with factors 1 where there
+// is none, so that lanes with different moments run the same operations.
+// first() and second() are the axes of f1 and f2, -1: the factor is 1.
+struct Moment3D {
+    static __device__ __forceinline__ int first(int j) { return j == 0 ? -1 : j <= 3 ? j - 1 : j <= 6 ? j - 4 : j == 8 ? 1 : 0; }
+    static __device__ __forceinline__ int second(int j) { return j <= 3 ? -1 : j <= 6 ? j - 4 : j == 7 ? 1 : 2; }
+    static __device__ __forceinline__ double half(int j) { return j >= 4 && j <= 6 ? 0.5 : 1.0; }
+};
 
 // P2M of every active leaf, one warp per cell: lane 10 a + j sums moment j of
 // source component a over the leaf's active particles in ascending index
@@ -370,15 +417,115 @@ p2m3d(Tree3D t, unsigned* err) {
     const int nc = t.info->n_cells;
     const int warps = gridDim.x * (blockDim.x >> 5);
     const int a = lane / 10, j = lane - 10 * (lane / 10);
+    const int i1 = Moment3D::first(j), i2 = Moment3D::second(j);
+    const double hf = Moment3D::half(j);
+    const double* src = a == 0 ? t.ax : a == 1 ? t.ay : t.az;
+    const double* p1 = i1 <= 0 ? t.px : i1 == 1 ? t.py : t.pz;
+    const double* p2 = i2 <= 0 ? t.px : i2 == 1 ? t.py : t.pz;
     for (int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < nc; c += warps) {
         double m = 0.0;
         if (t.c_chmask[c] == 0 && t.c_active[c] && lane < 30) {
-            const double xc = t.c_x[c], yc = t.c_y[c], zc = t.c_z[c];
-            const double* src = a == 0 ? t.ax : a == 1 ? t.ay : t.az;
+            const double c1 = i1 <= 0 ? t.c_x[c] : i1 == 1 ? t.c_y[c] : t.c_z[c];
+            const double c2 = i2 <= 0 ? t.c_x[c] : i2 == 1 ? t.c_y[c] : t.c_z[c];
             for (int s = t.c_lo[c]; s < t.c_hi[c]; ++s) {
                 if (!t.pact[s]) continue;
-                p2m_term(m, j, src[s], xc - t.px[s], yc - t.py[s], zc - t.pz[s]);
+                m += src[s] * (i1 < 0 ? 1.0 : c1 - p1[s]) * (i2 < 0 ? 1.0 : c2 - p2[s]) * hf;
             }
+        }
+        if (lane < 30) t.mom[(size_t)c * kMom3D + lane] = m;
+    }
+}
+
+// Leaves of at most kSmallLeaf particles, one warp per cell: the indices of
+// the leaf's range of `order` sorted (ascending index, the reference's
+// parIDList order), its particles gathered into the leaf order, and its P2M
+// from the copy the warp holds in shared memory. Replaces a radix sort by leaf
+// (five launches), the gather and p2m3d: 130 us of kernels on the 222,688-
+// particle ring, 560 on the 2,009,183-particle one; this kernel takes 32 and
+// 210.
+// Bound by its gathers (49 bytes a particle in the caller's order).
+constexpr int kSmallLeaf = 64;
+constexpr int kLeafWarps = 4;
+
+// Ascending over the warp; v of lane i is element i.
+__device__ __forceinline__ uint32_t warp_sort(uint32_t v, int lane) {
+    #pragma unroll
+    for (int k = 2; k <= 32; k <<= 1) {
+        #pragma unroll
+        for (int o = k >> 1; o > 0; o >>= 1) {
+            const uint32_t w = __shfl_xor_sync(0xffffffffu, v, o);
+            const bool up = (lane & k) == 0, low = (lane & o) == 0;
+            v = (up == low) ? min(v, w) : max(v, w);
+        }
+    }
+    return v;
+}
+
+__global__ void __launch_bounds__(32 * kLeafWarps)
+leaf_gather3d(Tree3D t, const uint32_t* __restrict__ order, const double* __restrict__ x,
+              const double* __restrict__ y, const double* __restrict__ z, const double* __restrict__ ax,
+              const double* __restrict__ ay, const double* __restrict__ az, const uint8_t* __restrict__ act,
+              unsigned* err) {
+    __shared__ double s_p[kLeafWarps][3][kSmallLeaf], s_a[kLeafWarps][3][kSmallLeaf];
+    if (fatal(err)) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int n = t.n, nc = t.info->n_cells;
+    const int a = lane / 10, j = lane - 10 * (lane / 10);
+    const int i1 = Moment3D::first(j), i2 = Moment3D::second(j);
+    const double hf = Moment3D::half(j);
+    const double* src = s_a[w][min(a, 2)];
+    const double* p1 = s_p[w][max(i1, 0)];
+    const double* p2 = s_p[w][max(i2, 0)];
+    for (int c = blockIdx.x * kLeafWarps + w; c < nc; c += gridDim.x * kLeafWarps) {
+        double m = 0.0;
+        if (t.c_chmask[c] == 0 && c > 0) {   // warp-uniform
+            const int lo = t.c_lo[c], cnt = t.c_hi[c] - lo;
+            if (cnt < 0 || cnt > kSmallLeaf || lo < 0 || lo + cnt > n) {
+                if (lane == 0) set_err(err, ERR_INDEX);
+                continue;
+            }
+            uint32_t v0 = lane < cnt ? order[lo + lane] : 0xffffffffu;
+            uint32_t v1 = lane + 32 < cnt ? order[lo + 32 + lane] : 0xffffffffu;
+            v0 = warp_sort(v0, lane);
+            if (cnt > 32) {                  // merge the two sorted halves
+                v1 = __shfl_xor_sync(0xffffffffu, warp_sort(v1, lane), 31);
+                const uint32_t lo32 = min(v0, v1), hi32 = max(v0, v1);
+                v0 = warp_sort(lo32, lane);
+                v1 = warp_sort(hi32, lane);
+            }
+            unsigned on[2] = {0u, 0u};
+            #pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int k = 32 * h + lane;
+                if (32 * h >= cnt) break;    // warp-uniform
+                const uint32_t i = h ? v1 : v0;
+                bool live = false;
+                if (k < cnt) {
+                    if (i >= (uint32_t)n) {
+                        set_err(err, ERR_INDEX);
+                    } else {
+                        const double q[6] = {x[i], y[i], z[i], ax[i], ay[i], az[i]};
+                        live = act[i] != 0;
+                        t.perm[lo + k] = i;
+                        t.px[lo + k] = s_p[w][0][k] = q[0];
+                        t.py[lo + k] = s_p[w][1][k] = q[1];
+                        t.pz[lo + k] = s_p[w][2][k] = q[2];
+                        t.ax[lo + k] = s_a[w][0][k] = q[3];
+                        t.ay[lo + k] = s_a[w][1][k] = q[4];
+                        t.az[lo + k] = s_a[w][2][k] = q[5];
+                        t.pact[lo + k] = live ? 1 : 0;
+                    }
+                }
+                on[h] = __ballot_sync(0xffffffffu, live);
+            }
+            __syncwarp();
+            const double c1 = i1 <= 0 ? t.c_x[c] : i1 == 1 ? t.c_y[c] : t.c_z[c];
+            const double c2 = i2 <= 0 ? t.c_x[c] : i2 == 1 ? t.c_y[c] : t.c_z[c];
+            for (int s = 0; s < cnt; ++s) {
+                if (!(((s < 32 ? on[0] : on[1]) >> (s & 31)) & 1u)) continue;   // warp-uniform
+                m += src[s] * (i1 < 0 ? 1.0 : c1 - p1[s]) * (i2 < 0 ? 1.0 : c2 - p2[s]) * hf;
+            }
+            __syncwarp();
         }
         if (lane < 30) t.mom[(size_t)c * kMom3D + lane] = m;
     }
@@ -390,6 +537,8 @@ p2m3d(Tree3D t, unsigned* err) {
 __device__ __forceinline__ void m2m3d_level(const Tree3D& t, int L) {
     const int lane = threadIdx.x & 31;
     const int a = lane / 10, j = lane - 10 * (lane / 10);
+    const int i1 = Moment3D::first(j), i2 = Moment3D::second(j);
+    const double hf = Moment3D::half(j);
     const int c0 = t.info->level_start[L], c1 = t.info->level_start[L + 1];
     const int warps = gridDim.x * (blockDim.x >> 5);
     for (int c = c0 + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < c1; c += warps) {
@@ -402,34 +551,29 @@ __device__ __forceinline__ void m2m3d_level(const Tree3D& t, int L) {
         for (int o = 0; o < 8; ++o) {
             if (!((mask >> o) & 1u)) continue;
             const int k = k0 + r++;
-            const double dx = xc - t.c_x[k], dy = yc - t.c_y[k], dz = zc - t.c_z[k];
             const double* ch = &t.mom[(size_t)k * kMom3D + 10 * a];
-            const double c_0 = __ldcg(&ch[0]), c_1 = __ldcg(&ch[1]), c_2 = __ldcg(&ch[2]), c_3 = __ldcg(&ch[3]);
-            const double cj = __ldcg(&ch[j]);
-            switch (j) {
-                case 0: m += cj; break;
-                case 1: m += cj + c_0 * dx; break;
-                case 2: m += cj + c_0 * dy; break;
-                case 3: m += cj + c_0 * dz; break;
-                case 4: m += cj + (c_0 * dx * dx * 0.5) + (c_1 * dx); break;
-                case 5: m += cj + (c_0 * dy * dy * 0.5) + (c_2 * dy); break;
-                case 6: m += cj + (c_0 * dz * dz * 0.5) + (c_3 * dz); break;
-                case 7: m += cj + (c_0 * dx * dy) + (c_1 * dy) + (c_2 * dx); break;
-                case 8: m += cj + (c_0 * dy * dz) + (c_2 * dz) + (c_3 * dy); break;
-                default: m += cj + (c_0 * dx * dz) + (c_1 * dz) + (c_3 * dx); break;
-            }
+            const double d[3] = {xc - t.c_x[k], yc - t.c_y[k], zc - t.c_z[k]};
+            const double d1 = i1 <= 0 ? d[0] : i1 == 1 ? d[1] : d[2], d2 = i2 <= 0 ? d[0] : i2 == 1 ? d[1] : d[2];
+            const double c_0 = __ldcg(&ch[0]), cj = __ldcg(&ch[j]);
+            const double f1 = __ldcg(&ch[1 + max(i1, 0)]), f2 = __ldcg(&ch[1 + max(i2, 0)]);
+            // cj + c_0 d1 d2 (1/2 on the diagonal) + first moments times the other axis
+            double v = cj;
+            if (j >= 1) v = v + c_0 * d1 * (j <= 3 ? 1.0 : d2) * hf;
+            if (j >= 4) v = v + f1 * d2;
+            if (j >= 7) v = v + f2 * d1;
+            m += v;
         }
         t.mom[(size_t)c * kMom3D + lane] = m;
     }
 }
 
 // M2M of levels depth-1 .. 1 in one cooperative launch.
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(512)
 m2m3d_coop(Tree3D t, unsigned* err) {
     const int depth = t.info->depth;
     for (int L = depth - 1; L >= 1; --L) {
         if (!block_fatal(err)) m2m3d_level(t, L);
-        grid_sync(t.gbar + 2, err);
+        if (L > 1) grid_sync_counter(t.gbar + 2, err);
     }
 }
 
@@ -509,6 +653,35 @@ __global__ void tc_keys3d(const double* __restrict__ x, const double* __restrict
             k |= tc_spread((uint32_t)ix) << d;
         }
         if (bad) set_err(err, ERR_RANGE);
+        key[i] = k;
+        idx[i] = (uint32_t)i;
+    }
+}
+
+// Key of the octree: the octants of the particle's cells of levels 1 .. 10,
+// found by walking down from the root with the reference's own centres
+// (fast3DFMM.cpp:652-655; an axis needs only its own bits). Runs of equal
+// prefixes are the octree's cells, in the order of the level-by-level build
+// (parents in order, octants 0..7 under a parent).
+__global__ void oct_keys3d(const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
+                           int n, const Geom3D* __restrict__ g, uint32_t* __restrict__ key,
+                           uint32_t* __restrict__ idx) {
+    const double cen[3] = {g->cen[0], g->cen[1], g->cen[2]}, root = g->root;
+    const double* p[3] = {x, y, z};
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        uint32_t k = 0;
+        #pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double v = p[d][i];
+            double c = cen[d], len = root;
+            #pragma unroll
+            for (int L = 1; L <= kTcLevels; ++L) {
+                const int bit = v > c;
+                k |= (uint32_t)bit << (3 * (kTcLevels - L) + d);
+                len = xmul(len, 0.5);
+                c = xadd(c, xmul(len, (double)bit - 0.5));
+            }
+        }
         key[i] = k;
         idx[i] = (uint32_t)i;
     }
@@ -594,9 +767,11 @@ __global__ void tc_bigl3d(const uint32_t* __restrict__ key, const uint32_t* __re
 // The levels of the cells particle j starts (first..last, 0 = none; bits
 // 16..23 and 24..31 of pinfo) and the per-tile counts of cells and leaves of
 // every level: rows 0..10 cells, rows 11..21 leaves, tiles columns.
+// deep (octree): set when a level-10 cell would need splitting, which is
+// ERR_DEPTH for the TreeCell (null).
 __global__ void __launch_bounds__(kTcTile)
 tc_cells3d(const uint32_t* __restrict__ key, uint32_t* __restrict__ pinfo, int n, uint32_t* __restrict__ tile_cnt,
-           int tiles, unsigned* err) {
+           int tiles, unsigned* deep, unsigned* err) {
     __shared__ unsigned s_c[kTcLevels + 1], s_l[kTcLevels + 1];
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         if (threadIdx.x <= kTcLevels) s_c[threadIdx.x] = s_l[threadIdx.x] = 0;
@@ -615,7 +790,10 @@ tc_cells3d(const uint32_t* __restrict__ key, uint32_t* __restrict__ pinfo, int n
                 if (exists) {
                     first = lvl;
                     last = min(kTcLevels, max(lvl, big + 1));
-                    if (big >= kTcLevels) set_err(err, ERR_DEPTH);   // a level-10 cell would need splitting
+                    if (big >= kTcLevels) {   // a level-10 cell would need splitting
+                        if (deep) atomicExch(deep, 1u);
+                        else set_err(err, ERR_DEPTH);
+                    }
                     for (int L = first; L <= last; ++L) atomicAdd(&s_c[L], 1u);
                     if (big < last) atomicAdd(&s_l[last], 1u);
                 }
@@ -668,10 +846,12 @@ tc_scan_rows3d(uint32_t* __restrict__ tile_cnt, int tiles, uint32_t* __restrict_
 // Level starts, depth and the root cell (treeCell.cpp:1117-1133); ERR_LEAF1
 // when a level-1 cell is a leaf and the tree goes deeper: the reference's
 // traversal asks for that leaf's children and throws (fmm3D.cpp:1286).
+template <bool OCT>
 __global__ void tc_totals3d(Tree3D t, const uint32_t* __restrict__ row_tot, const uint32_t* __restrict__ as,
                             unsigned* err) {
+    if (OCT && t.gbar[kDeepWord]) return;
     TreeInfo3D* info = t.info;
-    int cells = 1, depth = 0;
+    int cells = 1, depth = 0, leaves = 0;
     info->level_start[0] = 0;
     for (int L = 1; L < kMaxLevels3D + 2; ++L) {
         info->level_start[L] = cells;
@@ -679,27 +859,28 @@ __global__ void tc_totals3d(Tree3D t, const uint32_t* __restrict__ row_tot, cons
             const int c = (int)row_tot[L];
             if (c > 0) depth = L;
             cells += c;
+            leaves += (int)row_tot[kTcLevels + 1 + L];
         }
     }
     info->n_cells = cells;
-    info->n_leaves = 0;   // counted after the leaf sort
+    info->n_leaves = leaves;
     info->depth = depth;
     info->remaining = 0;
     info->scan_total = 0;
     info->p2p_pairs = 0;
     info->m2p_pairs = 0;
     if (cells > t.cap_cells) set_err(err, ERR_CELL_CAP);
-    if (depth > 1 && row_tot[kTcLevels + 1 + 1] > 0) set_err(err, ERR_LEAF1);
+    if (!OCT && depth > 1 && row_tot[kTcLevels + 1 + 1] > 0) set_err(err, ERR_LEAF1);
     const Geom3D* g = t.geom;
-    t.c_x[0] = xadd(g->piv[0], xmul(0.5, g->root));
-    t.c_y[0] = xadd(g->piv[1], xmul(0.5, g->root));
-    t.c_z[0] = xadd(g->piv[2], xmul(0.5, g->root));
+    t.c_x[0] = OCT ? g->cen[0] : xadd(g->piv[0], xmul(0.5, g->root));
+    t.c_y[0] = OCT ? g->cen[1] : xadd(g->piv[1], xmul(0.5, g->root));
+    t.c_z[0] = OCT ? g->cen[2] : xadd(g->piv[2], xmul(0.5, g->root));
     t.c_size[0] = g->root;
     t.c_npar[0] = t.n;
     t.c_parent[0] = -1;
     t.c_child0[0] = -1;   // lowered by tc_link3d (unsigned minimum: -1 = none)
     t.c_chmask[0] = 0;
-    t.c_active[0] = as[t.n] != 0 ? 1 : 0;
+    t.c_active[0] = OCT || as[t.n] != 0 ? 1 : 0;
     t.c_level[0] = 0;
     t.c_lo[0] = 0;
     t.c_hi[0] = t.n;
@@ -708,11 +889,12 @@ __global__ void tc_totals3d(Tree3D t, const uint32_t* __restrict__ row_tot, cons
 // Cell records of every particle's cell levels; cell index = level start +
 // scanned tile count + rank of the particle among the tile's emitters of that
 // level (warp ballots). code[c] = level-L Morton prefix | leaf << 31.
+template <bool OCT>
 __global__ void __launch_bounds__(kTcTile)
 tc_emit3d(Tree3D t, const uint32_t* __restrict__ key, const uint32_t* __restrict__ pinfo,
           const uint32_t* __restrict__ tile_cnt, int tiles, uint32_t* __restrict__ code_out, unsigned* err) {
     __shared__ int s_wc[kTcLevels + 1][kTcTile / 32];
-    if (block_fatal(err)) return;
+    if (block_fatal(err) || (OCT && t.gbar[kDeepWord])) return;
     const int n = t.n;
     const TreeInfo3D* info = t.info;
     const Geom3D* g = t.geom;
@@ -743,11 +925,27 @@ tc_emit3d(Tree3D t, const uint32_t* __restrict__ key, const uint32_t* __restrict
             }
             const bool leaf = L == last && big < last;
             const uint32_t pre = key[j] >> (3 * (kTcLevels - L));
-            const int ix = tc_compact(pre), iy = tc_compact(pre >> 1), iz = tc_compact(pre >> 2);
-            const double len = xdiv(root, ldexp(1.0, L));
-            t.c_x[ci] = xadd(g->piv[0], xmul(xadd(0.5, (double)ix), len));
-            t.c_y[ci] = xadd(g->piv[1], xmul(xadd(0.5, (double)iy), len));
-            t.c_z[ci] = xadd(g->piv[2], xmul(xadd(0.5, (double)iz), len));
+            double len;
+            if (OCT) {   // the reference's centres, level by level (fast3DFMM.cpp:652-655)
+                double cx = g->cen[0], cy = g->cen[1], cz = g->cen[2];
+                len = root;
+                for (int l = L - 1; l >= 0; --l) {
+                    const uint32_t o = pre >> (3 * l);
+                    len = xmul(len, 0.5);
+                    cx = xadd(cx, xmul(len, (double)(int)(o & 1u) - 0.5));
+                    cy = xadd(cy, xmul(len, (double)(int)((o >> 1) & 1u) - 0.5));
+                    cz = xadd(cz, xmul(len, (double)(int)((o >> 2) & 1u) - 0.5));
+                }
+                t.c_x[ci] = cx;
+                t.c_y[ci] = cy;
+                t.c_z[ci] = cz;
+            } else {
+                const int ix = tc_compact(pre), iy = tc_compact(pre >> 1), iz = tc_compact(pre >> 2);
+                len = xdiv(root, ldexp(1.0, L));
+                t.c_x[ci] = xadd(g->piv[0], xmul(xadd(0.5, (double)ix), len));
+                t.c_y[ci] = xadd(g->piv[1], xmul(xadd(0.5, (double)iy), len));
+                t.c_z[ci] = xadd(g->piv[2], xmul(xadd(0.5, (double)iz), len));
+            }
             t.c_size[ci] = len;
             t.c_lo[ci] = j;
             t.c_child0[ci] = -1;
@@ -761,12 +959,13 @@ tc_emit3d(Tree3D t, const uint32_t* __restrict__ key, const uint32_t* __restrict
 
 // Range, counts and activity of every cell (one search per cell), its parent
 // (the level L-1 cell of its prefix >> 3, by bisection over that level's
-// prefixes), the parent's child mask and first child; every leaf records
-// itself as the cell of its particles.
+// prefixes), the parent's child mask and first child; with `idx` every leaf
+// records itself as the cell of its particles (for a sort by leaf).
+template <bool OCT>
 __global__ void tc_link3d(Tree3D t, const uint32_t* __restrict__ key, const uint32_t* __restrict__ idx,
                           const uint32_t* __restrict__ as, const uint32_t* __restrict__ code, int max_par,
                           unsigned* err) {
-    if (fatal(err)) return;
+    if (fatal(err) || (OCT && t.gbar[kDeepWord])) return;
     const int nc = t.info->n_cells, n = t.n;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x + 1; c < nc; c += gridDim.x * blockDim.x) {
         const int L = t.c_level[c];
@@ -797,59 +996,16 @@ __global__ void tc_link3d(Tree3D t, const uint32_t* __restrict__ key, const uint
         t.c_parent[c] = p;
         atomicOr(&t.c_chmask[p], 1u << (pre & 7u));
         atomicMin(reinterpret_cast<unsigned*>(&t.c_child0[p]), (unsigned)c);
-        if (leaf)
+        if (leaf && idx)
             for (int k = lo; k < hi; ++k) t.pcell[idx[k]] = c;
     }
 }
 
 }  // namespace
 
-static cudaError_t leaves_upward3d(const double* x, const double* y, const double* z, const double* ax,
-                                   const double* ay, const double* az, const uint8_t* act, Tree3D& t, Scratch3D& s,
-                                   unsigned* err, cudaStream_t st, int* launches);
-
-// Tree build (bounding box, levels, leaf order) and upward pass, enqueued on st.
-cudaError_t build_tree3d(const double* x, const double* y, const double* z, const double* ax, const double* ay,
-                         const double* az, const uint8_t* act, const double center[3], double exp_pct, Tree3D& t,
-                         Scratch3D& s, double* bbox_partial, unsigned* err, cudaStream_t st, int* launches) {
-    const int n = t.n;
-    const int gridN = std::max(1, std::min(148 * 8, ceil_div(n, 256)));
-    cudaError_t e = cudaMemsetAsync(t.gbar, 0, sizeof(unsigned) * 8, st);
-    if (e != cudaSuccess) return e;
-    const int bb = std::max(1, std::min(kBBox3Blocks, ceil_div(n, 256)));
-    bbox3d<<<bb, 256, 0, st>>>(x, y, z, n, center[0], center[1], center[2], exp_pct, false, t.geom, bbox_partial,
-                                t.gbar + 6, err);
-    root3d<<<gridN, 256, 0, st>>>(t);
-    *launches += 2;
+static cudaError_t m2m3d(const Tree3D& t, unsigned* err, cudaStream_t st, int* launches) {
     int grid = 0;
-    e = launch_coop(octree_levels3d, kT3Threads, 0, st, 4, &grid, t, x, y, z, act, kCoopMaxBlocks3D, err);
-    if (e != cudaSuccess) return e;
-    *launches += 1;
-    return leaves_upward3d(x, y, z, ax, ay, az, act, t, s, err, st, launches);
-}
-
-// Particles in leaf order (stable: ascending index within a leaf, the
-// reference's parIDList order), leaf ranges, P2M and the M2M levels.
-static cudaError_t leaves_upward3d(const double* x, const double* y, const double* z, const double* ax,
-                                   const double* ay, const double* az, const uint8_t* act, Tree3D& t, Scratch3D& s,
-                                   unsigned* err, cudaStream_t st, int* launches) {
-    const int n = t.n;
-    const int gridN = std::max(1, std::min(148 * 8, ceil_div(n, 256)));
-    cudaError_t e = cudaSuccess;
-    int grid = 0;
-    leaf_keys3d<<<gridN, 256, 0, st>>>(t, s.key_a, s.val_a);
-    *launches += 1;
-    int bits = 1;
-    while ((1ll << bits) < (long long)t.cap_cells) ++bits;
-    uint32_t* keys = s.key_a;
-    uint32_t* vals = s.val_a;
-    e = radix_sort_pairs(&keys, &vals, s.key_b, s.val_b, n, bits, s.sort, err, st, launches);
-    if (e != cudaSuccess) return e;
-    leaf_ranges3d<<<gridN, 256, 0, st>>>(t, keys, vals, x, y, z, ax, ay, az, act, err);
-    count_leaves3d<<<148, 256, 0, st>>>(t);
-    p2m3d<<<148 * 8, 128, 0, st>>>(t, err);
-    *launches += 3;
-    e = launch_coop(m2m3d_coop, 128, 0, st, 8, &grid, t, err);
+    const cudaError_t e = launch_coop(m2m3d_coop, 512, 0, st, 2, &grid, t, err);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         for (int L = kMaxLevels3D - 1; L >= 1; --L) {
@@ -862,23 +1018,43 @@ static cudaError_t leaves_upward3d(const double* x, const double* y, const doubl
     return cudaGetLastError();
 }
 
-cudaError_t build_treecell3d(const double* x, const double* y, const double* z, const double* ax,
-                             const double* ay, const double* az, const uint8_t* act, int max_src, int max_par,
-                             double exp_pct, Tree3D& t, Scratch3D& s, double* bbox_partial, unsigned* err,
-                             cudaStream_t st, int* launches) {
+// Particles in leaf order by a radix sort on each particle's leaf (stable:
+// ascending index within a leaf, the reference's parIDList order), leaf
+// ranges, P2M and the M2M levels.
+static cudaError_t leaves_upward3d(const double* x, const double* y, const double* z, const double* ax,
+                                   const double* ay, const double* az, const uint8_t* act, Tree3D& t, Scratch3D& s,
+                                   unsigned* err, cudaStream_t st, int* launches) {
+    const int n = t.n;
+    const int gridN = std::max(1, std::min(148 * 8, ceil_div(n, 256)));
+    leaf_keys3d<<<gridN, 256, 0, st>>>(t, s.key_a, s.val_a);
+    *launches += 1;
+    int bits = 1;
+    while ((1ll << bits) < (long long)t.cap_cells) ++bits;
+    uint32_t* keys = s.key_a;
+    uint32_t* vals = s.val_a;
+    cudaError_t e = radix_sort_pairs(&keys, &vals, s.key_b, s.val_b, n, bits, s.sort, err, st, launches);
+    if (e != cudaSuccess) return e;
+    leaf_ranges3d<<<gridN, 256, 0, st>>>(t, keys, vals, x, y, z, ax, ay, az, act, err);
+    p2m3d<<<148 * 8, 128, 0, st>>>(t, err);
+    *launches += 2;
+    return m2m3d(t, err, st, launches);
+}
+
+// The flat construction from 30-bit keys (tc_keys3d or oct_keys3d in s.key_a,
+// indices in s.val_a): sort, cells of all levels, leaf order, upward pass.
+// Leaves of at most kSmallLeaf particles (max_par) are put in index order leaf
+// by leaf; larger ones by a second sort, since a warp cannot hold them.
+template <bool OCT>
+static cudaError_t build_flat3d(const double* x, const double* y, const double* z, const double* ax,
+                                const double* ay, const double* az, const uint8_t* act, int max_src, int max_par,
+                                Tree3D& t, Scratch3D& s, unsigned* err, cudaStream_t st, int* launches) {
     const int n = t.n;
     const int gridN = std::max(1, std::min(148 * 8, ceil_div(n, 256)));
     const int tiles = ceil_div(n, kTcTile);
     if (tiles > s.tc_tiles) return cudaErrorInvalidValue;
-    cudaError_t e = cudaMemsetAsync(t.gbar, 0, sizeof(unsigned) * 8, st);
-    if (e != cudaSuccess) return e;
-    const int bb = std::max(1, std::min(kBBox3Blocks, ceil_div(n, 256)));
-    bbox3d<<<bb, 256, 0, st>>>(x, y, z, n, 0.0, 0.0, 0.0, exp_pct, true, t.geom, bbox_partial, t.gbar + 6, err);
-    tc_keys3d<<<gridN, 256, 0, st>>>(x, y, z, n, t.geom, s.key_a, s.val_a, err);
-    *launches += 2;
     uint32_t* keys = s.key_a;
     uint32_t* vals = s.val_a;
-    e = radix_sort_pairs(&keys, &vals, s.key_b, s.val_b, n, 3 * kTcLevels, s.sort, err, st, launches);
+    cudaError_t e = radix_sort_pairs(&keys, &vals, s.key_b, s.val_b, n, 3 * kTcLevels, s.sort, err, st, launches);
     if (e != cudaSuccess) return e;
     tc_act3d<<<gridN, 256, 0, st>>>(act, vals, n, s.tc_act);
     *launches += 1;
@@ -886,17 +1062,73 @@ cudaError_t build_treecell3d(const double* x, const double* y, const double* z, 
     if (e != cudaSuccess) return e;
     *launches += 1;
     const int gt = std::max(1, std::min(tiles, 148 * 2));
+    const bool small = max_par <= kSmallLeaf;
     tc_bigl3d<<<gridN, 256, 0, st>>>(keys, s.tc_scan, n, max_src, max_par, s.tc_pinfo);
-    tc_cells3d<<<gt, kTcTile, 0, st>>>(keys, s.tc_pinfo, n, s.tc_tile, tiles, err);
+    tc_cells3d<<<gt, kTcTile, 0, st>>>(keys, s.tc_pinfo, n, s.tc_tile, tiles, OCT ? t.gbar + kDeepWord : nullptr, err);
     tc_scan_rows3d<<<2 * (kTcLevels + 1), 1024, 0, st>>>(s.tc_tile, tiles, s.tc_tot);
-    tc_totals3d<<<1, 1, 0, st>>>(t, s.tc_tot, s.tc_scan, err);
-    tc_emit3d<<<gt, kTcTile, 0, st>>>(t, keys, s.tc_pinfo, s.tc_tile, tiles, s.tc_code, err);
+    tc_totals3d<OCT><<<1, 1, 0, st>>>(t, s.tc_tot, s.tc_scan, err);
+    tc_emit3d<OCT><<<gt, kTcTile, 0, st>>>(t, keys, s.tc_pinfo, s.tc_tile, tiles, s.tc_code, err);
     const int gc = std::max(1, std::min(148 * 8, ceil_div(t.cap_cells, 256)));
-    tc_link3d<<<gc, 256, 0, st>>>(t, keys, vals, s.tc_scan, s.tc_code, max_par, err);
+    tc_link3d<OCT><<<gc, 256, 0, st>>>(t, keys, small ? nullptr : vals, s.tc_scan, s.tc_code, max_par, err);
     *launches += 6;
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
+    if (!small) return leaves_upward3d(x, y, z, ax, ay, az, act, t, s, err, st, launches);
+    if (OCT) {
+        int grid = 0;
+        e = launch_coop(octree_levels3d<true>, kT3Threads, 0, st, 4, &grid, t, x, y, z, act, vals, kCoopMaxBlocks3D,
+                        err);
+        if (e != cudaSuccess) return e;
+        *launches += 1;
+    }
+    leaf_gather3d<<<148 * 16, 32 * kLeafWarps, 0, st>>>(t, vals, x, y, z, ax, ay, az, act, err);
+    *launches += 1;
+    return m2m3d(t, err, st, launches);
+}
+
+// Tree build (bounding box, levels, leaf order) and upward pass, enqueued on
+// st. Leaves of at most kSmallLeaf particles: the flat construction; its keys
+// hold ten levels, and a deeper tree is found out on the device and built
+// level by level in the same call. Larger leaves (an unusual setting): level
+// by level.
+cudaError_t build_tree3d(const double* x, const double* y, const double* z, const double* ax, const double* ay,
+                         const double* az, const uint8_t* act, const double center[3], double exp_pct, Tree3D& t,
+                         Scratch3D& s, double* bbox_partial, unsigned* err, cudaStream_t st, int* launches) {
+    const int n = t.n;
+    cudaError_t e = cudaMemsetAsync(t.gbar, 0, sizeof(unsigned) * 8, st);
+    if (e != cudaSuccess) return e;
+    const int bb = std::max(1, std::min(kBBox3Blocks, ceil_div(n, 256)));
+    bbox3d<<<bb, 256, 0, st>>>(x, y, z, n, center[0], center[1], center[2], exp_pct, false, t.geom, bbox_partial,
+                                t.gbar + 6, err);
+    *launches += 1;
+    if (t.leaf_cap - 1 <= kSmallLeaf) {
+        const int gridN = std::max(1, std::min(148 * 8, ceil_div(n, 256)));
+        oct_keys3d<<<gridN, 256, 0, st>>>(x, y, z, n, t.geom, s.key_a, s.val_a);
+        *launches += 1;
+        return build_flat3d<true>(x, y, z, ax, ay, az, act, n, t.leaf_cap - 1, t, s, err, st, launches);
+    }
+    int grid = 0;
+    e = launch_coop(octree_levels3d<false>, kT3Threads, 0, st, 4, &grid, t, x, y, z, act, (uint32_t*)nullptr,
+                    kCoopMaxBlocks3D, err);
+    if (e != cudaSuccess) return e;
+    count_leaves3d<<<148, 256, 0, st>>>(t);
+    *launches += 2;
     return leaves_upward3d(x, y, z, ax, ay, az, act, t, s, err, st, launches);
+}
+
+cudaError_t build_treecell3d(const double* x, const double* y, const double* z, const double* ax,
+                             const double* ay, const double* az, const uint8_t* act, int max_src, int max_par,
+                             double exp_pct, Tree3D& t, Scratch3D& s, double* bbox_partial, unsigned* err,
+                             cudaStream_t st, int* launches) {
+    const int n = t.n;
+    const int gridN = std::max(1, std::min(148 * 8, ceil_div(n, 256)));
+    cudaError_t e = cudaMemsetAsync(t.gbar, 0, sizeof(unsigned) * 8, st);
+    if (e != cudaSuccess) return e;
+    const int bb = std::max(1, std::min(kBBox3Blocks, ceil_div(n, 256)));
+    bbox3d<<<bb, 256, 0, st>>>(x, y, z, n, 0.0, 0.0, 0.0, exp_pct, true, t.geom, bbox_partial, t.gbar + 6, err);
+    tc_keys3d<<<gridN, 256, 0, st>>>(x, y, z, n, t.geom, s.key_a, s.val_a, err);
+    *launches += 2;
+    return build_flat3d<false>(x, y, z, ax, ay, az, act, max_src, max_par, t, s, err, st, launches);
 }
 
 }  // namespace vpm
