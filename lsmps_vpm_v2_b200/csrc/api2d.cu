@@ -107,7 +107,7 @@ int Ctx::reserve2d(int n, int cap_cells, int P, long long cap_l1, long long cap_
     size_t o_op = L.take<double2>((size_t)49 * (P + 1) * P);
     const int dlev = dense_levels_for(n);
     size_t o_dense = L.take<int32_t>((size_t)dense_entries(dlev));
-    size_t o_mixed = L.take<char>(mixed_bytes(n, cap_cells, P));
+    size_t o_mixed = L.take<char>(mixed_bytes(cap_cells));
 
     drop_graph();
     if (arena2d) cudaFree(arena2d);
@@ -161,12 +161,8 @@ int Ctx::reserve2d(int n, int cap_cells, int P, long long cap_l1, long long cap_
     ex2.coef = (double*)P_(o_coef);
     ex2.op = (double2*)P_(o_op);
     coef_P = -1;  // the new arena holds no coefficients yet
-    mixed_base = P_(o_mixed);
-    {
-        const size_t r0 = ((sizeof(double4) * (size_t)n + 1023) & ~(size_t)1023);
-        tc_rows = (float*)((char*)mixed_base + r0);
-        tc_ops = (float*)((char*)tc_rows + ((m2l_tc_rows_bytes(cap_cells) + 1023) & ~(size_t)1023));
-    }
+    tc_rows = (float*)P_(o_mixed);
+    tc_ops = (float*)((char*)tc_rows + ((m2l_tc_rows_bytes(cap_cells) + 1023) & ~(size_t)1023));
     cap.n = n; cap.cells = cap_cells; cap.P = P; cap.l1 = cap_l1; cap.l3 = cap_l3;
     return VPM_OK;
 }
@@ -236,8 +232,8 @@ int Ctx::enqueue2d(const double* x, const double* y, const double* q, const uint
         // One captured graph: the near field (lists 1/3, P2P) runs on the side
         // stream concurrently with lists 2/4 and the far field (P2M, M2M, M2L,
         // L2L); M2P follows lists 2/4 on the third stream once the upward pass
-        // and list 3 are done (the mixed form: list 3 from the slots, the few
-        // leaves that outgrew them after the CSR on the fourth stream; its M2L
+        // and list 3 are done (list 3 from the slots, the few leaves that
+        // outgrew them after the CSR on the fourth stream; the mixed form's M2L
         // of the levels below the large cells also runs on the third stream,
         // beside the large cells' M2M loop); L2P then adds the M2P and
         // near-field sums and writes the output.
@@ -248,31 +244,29 @@ int Ctx::enqueue2d(const double* x, const double* y, const double* q, const uint
             VPM_CUDA_TRY(gather_strengths2d(tree, q, d_err, st, &launches));
             VPM_CUDA_TRY(cudaEventRecord(ev_qg, st));
         }
-        const bool slots = p.precision != VPM_PREC_FP64 && int_lists_slotted(lists);
+        const bool slots = int_lists_slotted(lists);
+        auto near = [&](cudaStream_t on, int from) {
+            return (p.precision != VPM_PREC_FP64 ? fmm2d_p2p_f32 : fmm2d_p2p_f64)(
+                tree, lists, ex2, near_x, near_y, 0, 0.0, 0.0, d_err, on, &launches, true, from);
+        };
         if (slots) {
-            // the mixed near field and M2P start from the list slots; the CSR
+            // the near field and M2P start from the list slots; the CSR
             // (for the few leaves whose lists outgrew their slots) is built on
             // a third side stream meanwhile
             VPM_CUDA_TRY(build_int_slots2d(tree, lists, p.eps, d_err, side, &launches));
             VPM_CUDA_TRY(cudaEventRecord(ev_slots, side));
             if (deferred) VPM_CUDA_TRY(cudaStreamWaitEvent(side, ev_qg, 0));
-            VPM_CUDA_TRY(fmm2d_p2p_f32(tree, lists, ex2, near_x, near_y, 0, 0.0, 0.0, d_err, side, &launches, true,
-                                       kP2PListSlots));
+            VPM_CUDA_TRY(near(side, kP2PListSlots));
             VPM_CUDA_TRY(cudaStreamWaitEvent(side3, ev_slots, 0));
             VPM_CUDA_TRY(build_int_csr2d(tree, lists, ts.scan, p.eps, d_err, side3, &launches));
             VPM_CUDA_TRY(cudaEventRecord(ev_l13, side3));
             if (deferred) VPM_CUDA_TRY(cudaStreamWaitEvent(side3, ev_qg, 0));
-            VPM_CUDA_TRY(fmm2d_p2p_f32(tree, lists, ex2, near_x, near_y, 0, 0.0, 0.0, d_err, side3, &launches, true,
-                                       kP2PListSpill));
+            VPM_CUDA_TRY(near(side3, kP2PListSpill));
         } else {
             VPM_CUDA_TRY(build_int_lists2d(tree, lists, ts.scan, p.eps, d_err, side, &launches));
             VPM_CUDA_TRY(cudaEventRecord(ev_l13, side));
             if (deferred) VPM_CUDA_TRY(cudaStreamWaitEvent(side, ev_qg, 0));
-            if (p.precision != VPM_PREC_FP64)
-                VPM_CUDA_TRY(fmm2d_p2p_f32(tree, lists, ex2, near_x, near_y, 0, 0.0, 0.0, d_err, side, &launches, true));
-            else
-                VPM_CUDA_TRY(fmm2d_p2p_f64_tma(tree, lists, ex2, (double4*)mixed_base, near_x, near_y, 0, 0.0, 0.0,
-                                               d_err, side, &launches, p.max_par, true));
+            VPM_CUDA_TRY(near(side, kP2PListCsr));
         }
         VPM_CUDA_TRY(cudaEventRecord(join2, side));
         VPM_CUDA_TRY(cudaStreamWaitEvent(side2, fork2, 0));
@@ -360,8 +354,7 @@ int Ctx::enqueue2d(const double* x, const double* y, const double* q, const uint
         } else if (p.precision != VPM_PREC_FP64) {
             VPM_CUDA_TRY(fmm2d_p2p_f32(tree, lists, ex2, o0, o1, velocity, uinf, vinf, d_err, st, &launches));
         } else {
-            VPM_CUDA_TRY(fmm2d_p2p_f64_tma(tree, lists, ex2, (double4*)mixed_base, o0, o1, velocity, uinf, vinf, d_err,
-                                           st, &launches, p.max_par));
+            VPM_CUDA_TRY(fmm2d_p2p_f64(tree, lists, ex2, o0, o1, velocity, uinf, vinf, d_err, st, &launches));
         }
         if (int r = record(8)) return r;
     }

@@ -41,8 +41,8 @@ struct HostTree2D {
     std::vector<int> by_id;
 };
 
-// Size of the mixed-precision work area inside the 2D arena.
-size_t mixed_bytes(int n, int cap_cells, int P);
+// Size of the tensor-core work area inside the 2D arena.
+size_t mixed_bytes(int cap_cells);
 
 struct Ctx {
     int device = 0;
@@ -81,7 +81,6 @@ struct Ctx {
     TreeScratch2D ts{};
     Lists2D lists{};
     Expansions2D ex2{};
-    void* mixed_base = nullptr;
     float* tc_rows = nullptr;   // tensor-core M2L: scaled TF32 multipole rows
     float* tc_ops = nullptr;    //                  list-2 operators (hi, lo)
     int coef_P = -1, coef_binom = -1;
@@ -217,11 +216,10 @@ struct Ctx {
 cudaError_t fmm2d_p2p_f32(const Tree2D& t, const Lists2D& l, const Expansions2D& e, double* out0, double* out1,
                           int velocity, double u_inf, double v_inf, unsigned* err, cudaStream_t st, int* launches,
                           bool near_only = false, int lists = kP2PListCsr);
-// FP64 P2P on an AoS copy of the particles (`aos`, n entries); kernel choice as
-// for fmm2d_p2p_f32.
-cudaError_t fmm2d_p2p_f64_tma(const Tree2D& t, const Lists2D& l, const Expansions2D& e, double4* aos, double* out0,
-                              double* out1, int velocity, double u_inf, double v_inf, unsigned* err, cudaStream_t st,
-                              int* launches, int max_par, bool near_only = false);
+// FP64 P2P (near2d_f64), arguments as for fmm2d_p2p_f32.
+cudaError_t fmm2d_p2p_f64(const Tree2D& t, const Lists2D& l, const Expansions2D& e, double* out0, double* out1,
+                          int velocity, double u_inf, double v_inf, unsigned* err, cudaStream_t st, int* launches,
+                          bool near_only = false, int lists = kP2PListCsr);
 // Far field (M2P + L2P) plus the near field nx/ny (tree order), written in the
 // caller's order (field or velocity). With m2p_done the list-3 sums are
 // already in e.fx/e.fy (fmm2d_m2p) and only L2P is added (same result).
@@ -233,7 +231,5 @@ cudaError_t fmm2d_eval_combine(const Tree2D& t, const Lists2D& l, Expansions2D& 
 // the leaves whose list outgrew them, the spill pass takes exactly those).
 cudaError_t fmm2d_m2p(const Tree2D& t, const Lists2D& l, Expansions2D& e, int P, unsigned* err, cudaStream_t st,
                       int* launches, int lists = kP2PListCsr);
-cudaError_t fmm2d_p2p_out(const Tree2D& t, const Lists2D& l, const Expansions2D& e, double* out0, double* out1,
-                          int velocity, double u_inf, double v_inf, unsigned* err, cudaStream_t st, int* launches);
 
 }  // namespace vpm

@@ -269,7 +269,8 @@ cudaError_t fmm2d_m2l_only(const Tree2D& t, const Lists2D& l, Expansions2D& e, i
 cudaError_t fmm2d_l2l(const Tree2D& t, Expansions2D& e, int P, unsigned* err, cudaStream_t st, int* launches);
 cudaError_t fmm2d_eval(const Tree2D& t, const Lists2D& l, Expansions2D& e, int P, unsigned* err, cudaStream_t st,
                        int* launches);
-cudaError_t fmm2d_p2p(const Tree2D& t, const Lists2D& l, const Expansions2D& e, double* ex, double* ey,
-                      unsigned* err, cudaStream_t st, int* launches);
+// Potential over list 1 plus the far field in e.fx, into out (caller order).
+cudaError_t fmm2d_p2p_potential(const Tree2D& t, const Lists2D& l, const Expansions2D& e, double* out, unsigned* err,
+                                cudaStream_t st, int* launches);
 
 }  // namespace vpm

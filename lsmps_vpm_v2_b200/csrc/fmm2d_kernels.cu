@@ -21,7 +21,7 @@
 //                 (fmm2D.cpp:1040-1066) and L2P (fmm2D.cpp:1076-1093), warp per
 //                 leaf; the combine pass adds the near field and writes the
 //                 output in the caller's order.
-//   fmm2d_p2p_f64_tma, fmm2d_p2p_f32  near field over list 1, j != i
+//   fmm2d_p2p_f64, fmm2d_p2p_f32, fmm2d_p2p_potential  near field over list 1, j != i
 //                 (fmm2D.cpp:135-179): FP64 warp kernel for the plain form,
 //                 packed FP32 tiles for the mixed forms.
 #include "fmm2d.cuh"
@@ -587,8 +587,6 @@ eval2d(Tree2D t, Lists2D l, const double2* __restrict__ a, const double2* __rest
 
 // ---- P2P over list 1 --------------------------------------------------------
 
-constexpr int kP2PThreads = 128;
-
 // Writes one target's total field (near + far) in the caller's order; with
 // fx == nullptr (near field computed concurrently with the far field) the
 // near field alone, in tree order, into out0/out1.
@@ -614,83 +612,6 @@ __device__ __forceinline__ void p2p_store(const Tree2D& t, int ti, double ex, do
     }
 }
 
-// One block per leaf (grid-stride). With H = ceil(T/2), thread (t, split)
-// owns targets t and t + H and the sources split, split + ns, ... of every
-// list-1 cell (ns = 128 / H), so each source load serves two targets. Sources
-// come straight from global memory (L1-resident, nearly warp-uniform
-// addresses); the j == i exclusion is only tested inside the target's own
-// leaf. Partial sums are combined in a fixed order.
-__global__ void __launch_bounds__(kP2PThreads)
-p2p2d(Tree2D t, Lists2D l, const double* __restrict__ fx, const double* __restrict__ fy, double* __restrict__ out0,
-      double* __restrict__ out1, int velocity, double u_inf, double v_inf, unsigned* err) {
-    __shared__ double s_px[2][kP2PThreads], s_py[2][kP2PThreads];
-    if (fatal(err)) return;
-    const int nl = t.info->n_leaves;
-    const double* __restrict__ px = t.px;
-    const double* __restrict__ py = t.py;
-    const double* __restrict__ pq = t.pq;
-    for (int li = blockIdx.x; li < nl; li += gridDim.x) {
-        const int c = t.leaf_cells[li];
-        const int lo = t.c_lo[c], hi = t.c_hi[c];
-        const uint32_t o1 = l.l1_off[li], e1 = l.l1_off[li + 1];
-        for (int tb = lo; tb < hi; tb += 2 * kP2PThreads) {
-            const int T = min(2 * kP2PThreads, hi - tb);
-            const int H = (T + 1) >> 1;
-            const int ns = kP2PThreads / H;
-            const int tt = threadIdx.x % H, split = threadIdx.x / H;
-            const bool on = split < ns;
-            const int ta = tb + tt, tbb = tb + tt + H;
-            const bool hasb = tt + H < T;
-            const double xa = px[ta], ya = py[ta];
-            const double xb = hasb ? px[tbb] : xa, yb = hasb ? py[tbb] : ya;
-            double exa = 0.0, eya = 0.0, exb = 0.0, eyb = 0.0;
-            if (on) {
-                for (uint32_t k = o1; k < e1; ++k) {
-                    const int sc = l.l1_src[k];
-                    const int s_hi = t.c_hi[sc];
-                    if (sc != c) {
-                        for (int j = t.c_lo[sc] + split; j < s_hi; j += ns) {
-                            const double sx = __ldg(px + j), sy = __ldg(py + j), sq = __ldg(pq + j);
-                            const double dxa = xa - sx, dya = ya - sy, dxb = xb - sx, dyb = yb - sy;
-                            const double fa = sq * rcp_nr(fma(dxa, dxa, dya * dya));
-                            const double fb = sq * rcp_nr(fma(dxb, dxb, dyb * dyb));
-                            exa = fma(fa, dxa, exa);
-                            eya = fma(fa, dya, eya);
-                            exb = fma(fb, dxb, exb);
-                            eyb = fma(fb, dyb, eyb);
-                        }
-                    } else {
-                        for (int j = t.c_lo[sc] + split; j < s_hi; j += ns) {
-                            const double sx = __ldg(px + j), sy = __ldg(py + j), sq = __ldg(pq + j);
-                            const double dxa = xa - sx, dya = ya - sy, dxb = xb - sx, dyb = yb - sy;
-                            const double fa = (j == ta) ? 0.0 : sq * rcp_nr(fma(dxa, dxa, dya * dya));
-                            const double fb = (j == tbb) ? 0.0 : sq * rcp_nr(fma(dxb, dxb, dyb * dyb));
-                            exa = fma(fa, dxa, exa);
-                            eya = fma(fa, dya, eya);
-                            exb = fma(fb, dxb, exb);
-                            eyb = fma(fb, dyb, eyb);
-                        }
-                    }
-                }
-            }
-            if (on && split > 0) {
-                s_px[0][threadIdx.x] = exa; s_py[0][threadIdx.x] = eya;
-                s_px[1][threadIdx.x] = exb; s_py[1][threadIdx.x] = eyb;
-            }
-            __syncthreads();
-            if (split == 0) {
-                for (int s = 1; s < ns; ++s) {
-                    exa += s_px[0][s * H + tt]; eya += s_py[0][s * H + tt];
-                    exb += s_px[1][s * H + tt]; eyb += s_py[1][s * H + tt];
-                }
-                p2p_store(t, ta, exa, eya, fx, fy, out0, out1, velocity, u_inf, v_inf, err);
-                if (hasb) p2p_store(t, tbb, exb, eyb, fx, fy, out0, out1, velocity, u_inf, v_inf, err);
-            }
-            __syncthreads();
-        }
-    }
-}
-
 // ---- mixed form: FP32 near field ---------------------------------------------
 
 // FP32 reciprocal (hardware approximation, ~1 ulp) of the mixed near field.
@@ -701,402 +622,261 @@ __device__ __forceinline__ float rcp_approx(float a) {
 }
 
 
-// ---- TMA-staged P2P (bulk copies into shared memory) ------------------------------
+constexpr int kP2PMeta = 64;   // list-1 cells staged per leaf at a time
 
-constexpr int kStageCells = 64;  // list-1 cells of one leaf held in the stage descriptor
+// ---- FP64 near field ---------------------------------------------------------
 
-struct StageCell {
-    int start, end;  // staged slots [start, end)
-    float ox, oy;    // c_src - c_tgt (FP64 difference rounded once)
+// The plain form's field and the potential over list 1 (fmm2D.cpp:135-179 and
+// 77-122), one warp per leaf. A chunk of T <= 192 of the leaf's targets is
+// spread over H lanes with M = ceil(T / H) targets each, and the ns = 32 / H
+// lane groups take every ns-th source of the leaf's list-1 cells, which form
+// one flat sequence staged 64 at a time in shared memory (loaded a step
+// ahead). M is picked per chunk for the fewest lane-cycles (near_shape): lanes
+// without a target and slots without one are what the FP64 pipe loses, and a
+// staged source costs the SM 24 bytes a lane of its 128 a cycle, so few
+// targets per lane would be bound by shared memory. The pair itself is ten
+// FP64 operations. j == i is tested only in the steps that hold the leaf's own
+// cell (the reference's NaN of two coincident particles stays). Partial sums
+// are added over the lane groups in a fixed order.
+// 242 M pairs (778,377-particle boundary layer, caps 50/75): @NEW64@ us; the
+// kernel before took four targets per lane, cell by cell from global memory,
+// 379 us and a 13 us copy of the particles.
+constexpr int kNear64Warps = 4;
+constexpr int kNear64Stage = 64;
+constexpr int kNear64MaxM = 6;
+constexpr int kNear64Chunk = 32 * kNear64MaxM;
+
+struct Near64Warp {
+    union {
+        struct {
+            double2 xy[kNear64Stage];
+            double q[kNear64Stage];
+        } st;
+        double red[2 * kNear64MaxM][32];
+    };
+    int2 meta[kP2PMeta];       // first particle and size of each list-1 cell
+    int cs[kP2PMeta + 1];      // its flat start, then the total
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-// Bounded wait on the phase with the given parity; false on timeout.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
-    const uint32_t a = smem_u32(bar);
-    for (long long i = 0; i < kSpinLimit; ++i) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(a), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-// One bulk copy global -> this CTA's shared memory, completing on `bar`.
-// Both addresses 16-byte aligned, size a multiple of 16 (float4 elements).
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
-
-// Per-precision pieces of the TMA-staged P2P.
-struct P2PF64 {
-    using Elem = double4;  // (x, y, q, -) in FP64, absolute coordinates
-    using Acc = double;
-    static __device__ __forceinline__ void shift(Elem&, float, float) {}
-    static __device__ __forceinline__ double inv(double r2) { return rcp_nr(r2); }
-    static constexpr int kWarps = 4;
-    static constexpr int kMinBlocks = 5;   // <= 102 registers
-};
-
-// Stage the list-1 sources of leaf `li` into `buf` with one bulk copy per
-// source cell (one thread). Returns the staged slot count, or -1 when the
-// leaf does not fit (the barrier is still armed, with zero bytes, so its
-// phase completes); cells[k] receives each cell's slot range and its centre
-// offset relative to the target leaf (FP64 difference rounded once).
-template <class Elem>
-__device__ int stage_leaf(const Tree2D& t, const Lists2D& l, const Elem* src, int li, Elem* buf, int cap,
-                          StageCell* cells, uint64_t* bar) {
-    const int c = t.leaf_cells[li];
-    const double ccx = t.c_cx[c], ccy = t.c_cy[c];
-    const uint32_t o1 = l.l1_off[li], e1 = l.l1_off[li + 1];
-    int total = 0;
-    bool fits = (int)(e1 - o1) <= kStageCells;
-    if (fits) {
-        for (uint32_t k = o1; k < e1; ++k) {
-            const int sc = l.l1_src[k];
-            total += t.c_hi[sc] - t.c_lo[sc];
-        }
-        fits = total <= cap;
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_arrive_expect_tx(bar, fits ? (unsigned)(total * sizeof(Elem)) : 0u);
-    if (!fits) return -1;
-    int pos = 0, kk = 0;
-    for (uint32_t k = o1; k < e1; ++k, ++kk) {
-        const int sc = l.l1_src[k];
-        const int lo = t.c_lo[sc], hi = t.c_hi[sc];
-        cells[kk].start = pos;
-        cells[kk].end = pos + (hi - lo);
-        cells[kk].ox = (float)(t.c_cx[sc] - ccx);
-        cells[kk].oy = (float)(t.c_cy[sc] - ccy);
-        bulk_g2s(buf + pos, src + lo, (unsigned)((hi - lo) * sizeof(Elem)), bar);
-        pos += hi - lo;
-    }
-    return total;
-}
-
-constexpr int kTPT = 4;  // targets per thread in the TMA P2P
-
-// Pair loop of one thread over source slots [j0, j1) (step ns) for kTPT
-// targets; slot self[k] is excluded for target k (-1: none). FP32 sums are
-// flushed into the FP64 accumulators every 64 sources.
-template <class Tr>
-__device__ __forceinline__ void pair_loop4(const typename Tr::Elem* __restrict__ buf, int j0, int j1, int ns,
-                                           const double* tx, const double* ty, const int* self, double* ex,
-                                           double* ey) {
-    using A = typename Tr::Acc;
-    A x[kTPT], y[kTPT];
+// Targets per lane of a chunk of T: the least (10 M + 3) / ns, ten operations
+// per pair and about three for a step.
+__device__ __forceinline__ int near_shape(int T) {
+    int best = kNear64MaxM, bc = 10 * kNear64MaxM + 3, bn = 32 / ((T + kNear64MaxM - 1) / kNear64MaxM);
     #pragma unroll
-    for (int k = 0; k < kTPT; ++k) { x[k] = (A)tx[k]; y[k] = (A)ty[k]; }
-    const bool has_self = self[0] >= 0 || self[1] >= 0 || self[2] >= 0 || self[3] >= 0;
-    for (int jb = j0; jb < j1; jb += 64 * ns) {
-        const int je = min(j1, jb + 64 * ns);
-        A px[kTPT], py[kTPT];
+    for (int M = kNear64MaxM - 1; M >= 1; --M) {
+        const int H = (T + M - 1) / M;
+        if (H > 32) break;
+        const int ns = 32 / H, c = 10 * M + 3;
+        if (c * bn < bc * ns) {
+            best = M;
+            bc = c;
+            bn = ns;
+        }
+    }
+    return best;
+}
+
+// Staged sources s0, s0 + ns, ... below cnt onto the lane's M targets; SELF:
+// flat source self[k] is target k itself. POT: sums q log(r^2) in ex.
+template <int M, bool POT, bool SELF>
+__device__ __forceinline__ void near64_pairs(const double2* xy, const double* q, int s0, int cnt, int ns,
+                                             const double* x, const double* y, const int* self, double* ex,
+                                             double* ey) {
+    if (s0 >= cnt) return;
+    double2 pn = xy[s0];   // the next source, loaded while this one is applied
+    double wn = q[s0];
+    #pragma unroll 1
+    for (int s = s0; s < cnt; s += ns) {
+        const double2 p = pn;
+        const double w = wn;
+        const int sn = min(s + ns, kNear64Stage - 1);
+        pn = xy[sn];
+        wn = q[sn];
         #pragma unroll
-        for (int k = 0; k < kTPT; ++k) { px[k] = 0; py[k] = 0; }
-        if (!has_self) {
-            // the next source is loaded while this one is computed
-            typename Tr::Elem nv = jb < je ? buf[jb] : typename Tr::Elem{};
-            for (int j = jb; j < je; j += ns) {
-                const typename Tr::Elem sv = nv;
-                if (j + ns < je) nv = buf[j + ns];
-                const A sx = (A)sv.x, sy = (A)sv.y, sq = (A)sv.z;
-                #pragma unroll
-                for (int k = 0; k < kTPT; ++k) {
-                    const A dx = x[k] - sx, dy = y[k] - sy;
-                    const A f = sq * Tr::inv(dx * dx + dy * dy);
-                    px[k] += f * dx;
-                    py[k] += f * dy;
-                }
+        for (int k = 0; k < M; ++k) {
+            const double dx = x[k] - p.x, dy = y[k] - p.y;
+            const double r2 = fma(dx, dx, dy * dy);
+            if (POT) {
+                double v = w * log(r2);
+                if (SELF && s == self[k]) v = 0.0;
+                ex[k] += v;
+            } else {
+                double f = w * rcp_nr(r2);
+                if (SELF && s == self[k]) f = 0.0;
+                ex[k] = fma(f, dx, ex[k]);
+                ey[k] = fma(f, dy, ey[k]);
             }
+        }
+    }
+}
+
+template <int M, bool POT>
+__device__ __forceinline__ void near64_chunk(Near64Warp& sm, const Tree2D& t, const int32_t* __restrict__ src1, int c,
+                                             int lo, int n1, int tb, int T, const double* fx, const double* fy,
+                                             double* out0, double* out1, int velocity, double u_inf, double v_inf,
+                                             unsigned* err) {
+    const int lane = threadIdx.x & 31;
+    const int H = (T + M - 1) / M, ns = 32 / H;
+    const int tt = lane % H, split = lane / H;   // target k of this lane is chunk slot tt + k H
+    double x[M], y[M], ex[M], ey[M];
+    #pragma unroll
+    for (int k = 0; k < M; ++k) {
+        const int i = tt + k * H;
+        x[k] = t.px[tb + (i < T ? i : 0)];
+        y[k] = t.py[tb + (i < T ? i : 0)];
+        ex[k] = ey[k] = 0.0;
+    }
+    for (int seg = 0; seg < n1; seg += kP2PMeta) {
+        const int nseg = min(kP2PMeta, n1 - seg);
+        __syncwarp();
+        // ranges and flat starts of the segment's cells (two per lane), and
+        // the leaf's own flat range
+        int sz[2] = {0, 0}, inc[2];
+        bool own[2] = {false, false};
+        #pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int k = lane + 32 * h;
+            if (k < nseg) {
+                const int sc = src1[seg + k];
+                const int slo = t.c_lo[sc];
+                sz[h] = t.c_hi[sc] - slo;
+                own[h] = sc == c;
+                sm.meta[k] = make_int2(slo, sz[h]);
+            }
+            inc[h] = sz[h];
+        }
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int a0 = __shfl_up_sync(0xffffffffu, inc[0], o), a1 = __shfl_up_sync(0xffffffffu, inc[1], o);
+            if (lane >= o) {
+                inc[0] += a0;
+                inc[1] += a1;
+            }
+        }
+        const int tot0 = __shfl_sync(0xffffffffu, inc[0], 31);
+        const int total = tot0 + __shfl_sync(0xffffffffu, inc[1], 31);
+        const int start0 = inc[0] - sz[0], start1 = tot0 + inc[1] - sz[1];
+        if (lane < nseg) sm.cs[lane] = start0;
+        if (lane + 32 < nseg) sm.cs[lane + 32] = start1;
+        const unsigned b0 = __ballot_sync(0xffffffffu, own[0]), b1 = __ballot_sync(0xffffffffu, own[1]);
+        int own0 = -(1 << 30);
+        if (b0) own0 = __shfl_sync(0xffffffffu, start0, __ffs(b0) - 1);
+        else if (b1) own0 = __shfl_sync(0xffffffffu, start1, __ffs(b1) - 1);
+        const int self0 = own0 + (tb - lo) + tt;   // flat source that is target 0 of this lane
+        __syncwarp();
+        // per-lane walkers over the flat sequence: the lane stages flat sources
+        // cb + lane and cb + 32 + lane of step cb
+        int kw[2] = {0, 0}, ow[2] = {lane, lane + 32};
+        auto settle = [&](int h) {
+            while (kw[h] < nseg && ow[h] >= sm.meta[kw[h]].y) {
+                ow[h] -= sm.meta[kw[h]].y;
+                ++kw[h];
+            }
+        };
+        double vx[2], vy[2], vq[2];
+        auto fetch = [&](int h) {
+            vx[h] = vy[h] = vq[h] = 0.0;
+            if (kw[h] < nseg) {
+                const int j = sm.meta[kw[h]].x + ow[h];
+                vx[h] = t.px[j];
+                vy[h] = t.py[j];
+                vq[h] = t.pq[j];
+            }
+        };
+        #pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            settle(h);
+            fetch(h);
+        }
+        for (int cb = 0; cb < total; cb += kNear64Stage) {
+            #pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                sm.st.xy[lane + 32 * h] = make_double2(vx[h], vy[h]);
+                sm.st.q[lane + 32 * h] = vq[h];
+            }
+            __syncwarp();
+            #pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                ow[h] += kNear64Stage;
+                settle(h);
+                fetch(h);
+            }
+            const int cnt = min(kNear64Stage, total - cb);
+            const int s0 = split < ns ? split : cnt;
+            if (own0 < cb + kNear64Stage && own0 + (tb - lo) + T > cb) {   // warp-uniform
+                int self[M];
+                #pragma unroll
+                for (int k = 0; k < M; ++k) self[k] = tt + k * H < T ? self0 + k * H - cb : -1;
+                near64_pairs<M, POT, true>(sm.st.xy, sm.st.q, s0, cnt, ns, x, y, self, ex, ey);
+            } else {
+                near64_pairs<M, POT, false>(sm.st.xy, sm.st.q, s0, cnt, ns, x, y, nullptr, ex, ey);
+            }
+            __syncwarp();
+        }
+    }
+    // sum over the lane groups: lane tt + g H holds group g's parts of target slots tt + k H
+    __syncwarp();
+    #pragma unroll
+    for (int k = 0; k < M; ++k) {
+        sm.red[2 * k][lane] = ex[k];
+        if (!POT) sm.red[2 * k + 1][lane] = ey[k];
+    }
+    __syncwarp();
+    for (int i = lane; i < T; i += 32) {
+        const int k = i / H, l0 = i - k * H;
+        double sx = 0.0, sy = 0.0;
+        for (int g = 0; g < ns; ++g) {
+            sx += sm.red[2 * k][l0 + g * H];
+            if (!POT) sy += sm.red[2 * k + 1][l0 + g * H];
+        }
+        if (POT) {
+            const uint32_t orig = t.perm[tb + i];
+            if (orig >= (uint32_t)t.n) set_err(err, ERR_INDEX);
+            else out0[orig] = 0.5 * sx + fx[tb + i];
         } else {
-            for (int j = jb; j < je; j += ns) {
-                const typename Tr::Elem sv = buf[j];
-                const A sx = (A)sv.x, sy = (A)sv.y, sq = (A)sv.z;
-                #pragma unroll
-                for (int k = 0; k < kTPT; ++k) {
-                    const A dx = x[k] - sx, dy = y[k] - sy;
-                    A f = sq * Tr::inv(dx * dx + dy * dy);
-                    if (j == self[k]) f = 0;
-                    px[k] += f * dx;
-                    py[k] += f * dy;
-                }
-            }
+            p2p_store(t, tb + i, sx, sy, fx, fy, out0, out1, velocity, u_inf, v_inf, err);
         }
-        #pragma unroll
-        for (int k = 0; k < kTPT; ++k) { ex[k] += (double)px[k]; ey[k] += (double)py[k]; }
     }
+    __syncwarp();
 }
 
-// TMA-staged P2P. Each block walks its leaves (grid-stride) with two stage
-// buffers: while the block computes leaf i from one buffer, thread 0 has bulk
-// copies of leaf i+1's list-1 sources in flight into the other (one mbarrier
-// per buffer, bounded waits). After a stage lands the block adds each source
-// cell's centre offset (FP32 form: sources then share the target leaf's
-// frame), so the pair loop is one flat loop over the staged slots. Thread
-// (t, split) owns targets t and t + H (H = ceil(T/2)) and slots split,
-// split + ns, ... A leaf whose sources do not fit is computed from global
-// memory cell by cell.
-template <class Tr>
-__global__ void __launch_bounds__(kP2PThreads)
-p2p2d_tma(Tree2D t, Lists2D l, const typename Tr::Elem* __restrict__ src, const double* __restrict__ fx,
-          const double* __restrict__ fy, double* __restrict__ out0, double* __restrict__ out1, int velocity,
-          double u_inf, double v_inf, int cap, unsigned* err) {
-    using Elem = typename Tr::Elem;
-    extern __shared__ __align__(16) unsigned char p2p_sm[];
-    Elem* bufs = (Elem*)p2p_sm;                                        // [2][cap]
-    StageCell* scells = (StageCell*)(bufs + 2 * (size_t)cap);          // [2][kStageCells]
-    uint64_t* bars = (uint64_t*)(scells + 2 * kStageCells);            // [2]
-    int* s_count = (int*)(bars + 2);                                   // [2]
-    __shared__ double s_px[kTPT][kP2PThreads], s_py[kTPT][kP2PThreads];
+// List 1 from the CSR, or from the fixed slots (kP2PListSlots; the leaves
+// whose list outgrew them come in a second pass, kP2PListSpill, from the CSR).
+template <bool POT>
+__global__ void __launch_bounds__(32 * kNear64Warps, 3)
+near2d_f64(Tree2D t, Lists2D l, const double* __restrict__ fx, const double* __restrict__ fy,
+           double* __restrict__ out0, double* __restrict__ out1, int velocity, double u_inf, double v_inf, int lists,
+           unsigned* err) {
+    __shared__ Near64Warp sm[kNear64Warps];
     if (fatal(err)) return;
+    const int wib = threadIdx.x >> 5;
     const int nl = t.info->n_leaves;
-    if ((int)blockIdx.x >= nl) return;
-    if (threadIdx.x == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        s_count[0] = stage_leaf<Elem>(t, l, src, blockIdx.x, bufs, cap, scells, &bars[0]);
-    }
-    __syncthreads();
-    int iter = 0;
-    for (int li = blockIdx.x; li < nl; li += gridDim.x, ++iter) {
-        const int b = iter & 1;
-        const int nxt = li + gridDim.x;
-        if (threadIdx.x == 0 && nxt < nl)
-            s_count[b ^ 1] = stage_leaf<Elem>(t, l, src, nxt, bufs + (size_t)(b ^ 1) * cap, cap,
-                                              scells + (b ^ 1) * kStageCells, &bars[b ^ 1]);
-        const bool ok = mbar_wait(&bars[b], (iter >> 1) & 1);
-        if (!ok) set_err(err, ERR_TIMEOUT);
-        const int staged = s_count[b];
-        Elem* buf = bufs + (size_t)b * cap;
-        const StageCell* cells = scells + b * kStageCells;
+    for (int li = blockIdx.x * kNear64Warps + wib; li < nl; li += gridDim.x * kNear64Warps) {
+        const int32_t* src1;
+        int n1;
+        if (lists == kP2PListCsr) {
+            src1 = l.l1_src + l.l1_off[li];
+            n1 = (int)(l.l1_off[li + 1] - l.l1_off[li]);
+        } else {
+            const uint32_t cnt = l.l1_cnt[li];
+            const bool spill = cnt > (uint32_t)kListSlot1;
+            if (spill != (lists == kP2PListSpill)) continue;
+            src1 = spill ? l.l1_src + l.l1_off[li] : l.l1_slot + (size_t)li * kListSlot1;
+            n1 = spill ? (int)(l.l1_off[li + 1] - l.l1_off[li]) : (int)cnt;
+        }
         const int c = t.leaf_cells[li];
         const int lo = t.c_lo[c], hi = t.c_hi[c];
-        const double ccx = t.c_cx[c], ccy = t.c_cy[c];
-        const uint32_t o1 = l.l1_off[li], e1 = l.l1_off[li + 1];
-        const int ncell = (int)(e1 - o1);
-        // Own-leaf slot range, and the frame shift of the staged sources.
-        int own0 = -1;
-        if (staged >= 0 && ok) {
-            for (int kk = 0; kk < ncell; ++kk) {
-                const StageCell ci = cells[kk];
-                if (l.l1_src[o1 + kk] == c) own0 = ci.start;
-                for (int j = ci.start + threadIdx.x; j < ci.end; j += blockDim.x) Tr::shift(buf[j], ci.ox, ci.oy);
+        for (int tb = lo; tb < hi; tb += kNear64Chunk) {
+            const int T = min(kNear64Chunk, hi - tb);
+            switch (near_shape(T)) {
+#define VPM_NEAR_CASE(MM)                                                                                            \
+    case MM:                                                                                                         \
+        near64_chunk<MM, POT>(sm[wib], t, src1, c, lo, n1, tb, T, fx, fy, out0, out1, velocity, u_inf, v_inf, err);   \
+        break;
+                VPM_NEAR_CASE(1) VPM_NEAR_CASE(2) VPM_NEAR_CASE(3) VPM_NEAR_CASE(4) VPM_NEAR_CASE(5) VPM_NEAR_CASE(6)
+#undef VPM_NEAR_CASE
+                default: break;
             }
-        }
-        __syncthreads();
-        for (int tb = lo; tb < hi; tb += kTPT * kP2PThreads) {
-            const int T = min(kTPT * kP2PThreads, hi - tb);
-            const int H = (T + kTPT - 1) / kTPT;
-            const int ns = kP2PThreads / H;
-            const int tt = threadIdx.x % H, split = threadIdx.x / H;
-            const bool on = split < ns && ok;
-            int ti[kTPT];
-            double tx[kTPT], ty[kTPT], ex[kTPT], ey[kTPT];
-            #pragma unroll
-            for (int k = 0; k < kTPT; ++k) {
-                const int off = tt + k * H;
-                ti[k] = off < T ? tb + off : -1;
-                const Elem g = src[ti[k] >= 0 ? ti[k] : tb + tt];
-                tx[k] = g.x;
-                ty[k] = g.y;
-                ex[k] = 0.0;
-                ey[k] = 0.0;
-            }
-            if (on) {
-                if (staged >= 0) {
-                    int self[kTPT];
-                    #pragma unroll
-                    for (int k = 0; k < kTPT; ++k) self[k] = (own0 >= 0 && ti[k] >= 0) ? own0 + (ti[k] - lo) : -1;
-                    // Slots of the own leaf need the j == i test; the others do not.
-                    if (own0 >= 0) {
-                        const int own1 = own0 + (hi - lo);
-                        const int none[kTPT] = {-1, -1, -1, -1};
-                        pair_loop4<Tr>(buf, split, own0, ns, tx, ty, none, ex, ey);
-                        const int j0 = own0 + ((split - own0) % ns + ns) % ns;
-                        pair_loop4<Tr>(buf, j0, own1, ns, tx, ty, self, ex, ey);
-                        const int j2 = own1 + ((split - own1) % ns + ns) % ns;
-                        pair_loop4<Tr>(buf, j2, staged, ns, tx, ty, none, ex, ey);
-                    } else {
-                        pair_loop4<Tr>(buf, split, staged, ns, tx, ty, self, ex, ey);
-                    }
-                } else {
-                    for (int kk = 0; kk < ncell; ++kk) {
-                        const int sc = l.l1_src[o1 + kk];
-                        const int slo = t.c_lo[sc], shi = t.c_hi[sc];
-                        double sx = 0.0, sy = 0.0;
-                        if (sizeof(Elem) == sizeof(float4)) {
-                            sx = (double)(float)(t.c_cx[sc] - ccx);
-                            sy = (double)(float)(t.c_cy[sc] - ccy);
-                        }
-                        double tx2[kTPT], ty2[kTPT];
-                        int self[kTPT];
-                        #pragma unroll
-                        for (int k = 0; k < kTPT; ++k) {
-                            tx2[k] = tx[k] - sx;
-                            ty2[k] = ty[k] - sy;
-                            self[k] = (sc == c) ? ti[k] : -1;
-                        }
-                        pair_loop4<Tr>(src, slo + split, shi, ns, tx2, ty2, self, ex, ey);
-                    }
-                }
-            }
-            if (on && split > 0) {
-                #pragma unroll
-                for (int k = 0; k < kTPT; ++k) { s_px[k][threadIdx.x] = ex[k]; s_py[k][threadIdx.x] = ey[k]; }
-            }
-            __syncthreads();
-            if (split == 0 && ok) {
-                for (int s2 = 1; s2 < ns; ++s2) {
-                    #pragma unroll
-                    for (int k = 0; k < kTPT; ++k) { ex[k] += s_px[k][s2 * H + tt]; ey[k] += s_py[k][s2 * H + tt]; }
-                }
-                #pragma unroll
-                for (int k = 0; k < kTPT; ++k)
-                    if (ti[k] >= 0) p2p_store(t, ti[k], ex[k], ey[k], fx, fy, out0, out1, velocity, u_inf, v_inf, err);
-            }
-            __syncthreads();
-        }
-    }
-    // Copies are only issued for leaves this block then waits on; after a
-    // timed-out wait, wait once more (bounded) so no copy lands in freed
-    // shared memory.
-    if (threadIdx.x == 0 && iter > 0) {
-        const int last = iter - 1;
-        (void)mbar_wait(&bars[last & 1], (last >> 1) & 1);
-    }
-}
-
-// Warp-per-leaf P2P (the plain FP64 form's near field). Each warp owns one
-// leaf at a time (grid-stride over leaves), so no block-wide barrier sits in
-// the loop.
-// With H = ceil(T/4) lanes per split, lane (t, split) owns targets t, t+H,
-// t+2H, t+3H and the sources split, split + ns, ... (ns = 32/H) of every
-// list-1 cell, read straight from global memory (nearly warp-uniform
-// addresses, L1-resident). Split partials are summed in a fixed order through
-// a per-warp shared-memory tile.
-constexpr int kP2PMeta = 64;   // list-1 cells staged per leaf (longer lists read them directly)
-
-template <class Tr>
-__global__ void __launch_bounds__(32 * Tr::kWarps, Tr::kMinBlocks)
-p2p2d_warp(Tree2D t, Lists2D l, const typename Tr::Elem* __restrict__ src, const double* __restrict__ fx,
-           const double* __restrict__ fy, double* __restrict__ out0, double* __restrict__ out1, int velocity,
-           double u_inf, double v_inf, unsigned* err) {
-    using Elem = typename Tr::Elem;
-    __shared__ double s_red[Tr::kWarps][2 * kTPT][32];
-    // list-1 cells of the warp's leaf: first/last slot, FP32-rounded centre
-    // offset, loaded by the whole warp at once (one round of latency)
-    __shared__ int4 s_meta[Tr::kWarps][kP2PMeta];
-    if (fatal(err)) return;
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int nl = t.info->n_leaves;
-    const bool rel = sizeof(Elem) == sizeof(float4);
-    for (int li = blockIdx.x * Tr::kWarps + wib; li < nl; li += gridDim.x * Tr::kWarps) {
-        const int c = t.leaf_cells[li];
-        const int lo = t.c_lo[c], hi = t.c_hi[c];
-        const double ccx = t.c_cx[c], ccy = t.c_cy[c];
-        const uint32_t o1 = l.l1_off[li], e1 = l.l1_off[li + 1];
-        const int n1 = (int)(e1 - o1);
-        const bool meta = n1 <= kP2PMeta;
-        if (meta) {
-            for (int k = lane; k < n1; k += 32) {
-                const int sc = l.l1_src[o1 + k];
-                float ox = 0.f, oy = 0.f;
-                if (rel) {
-                    ox = (float)(t.c_cx[sc] - ccx);
-                    oy = (float)(t.c_cy[sc] - ccy);
-                }
-                s_meta[wib][k] = make_int4(t.c_lo[sc], sc == c ? -t.c_hi[sc] - 1 : t.c_hi[sc], __float_as_int(ox),
-                                           __float_as_int(oy));
-            }
-            __syncwarp();
-        }
-        for (int tb = lo; tb < hi; tb += kTPT * 32) {
-            const int T = min(kTPT * 32, hi - tb);
-            const int H = (T + kTPT - 1) / kTPT;
-            const int ns = 32 / H;
-            const int tt = lane % H, split = lane / H;
-            const bool on = split < ns;
-            int ti[kTPT];
-            double tx[kTPT], ty[kTPT], ex[kTPT], ey[kTPT];
-            #pragma unroll
-            for (int k = 0; k < kTPT; ++k) {
-                const int off = tt + k * H;
-                ti[k] = off < T ? tb + off : -1;
-                const Elem g = src[ti[k] >= 0 ? ti[k] : tb];
-                tx[k] = g.x;
-                ty[k] = g.y;
-                ex[k] = 0.0;
-                ey[k] = 0.0;
-            }
-            if (on) {
-                for (uint32_t kk = o1; kk < e1; ++kk) {
-                    int slo, shi;
-                    bool own;
-                    double sx = 0.0, sy = 0.0;
-                    if (meta) {
-                        const int4 m = s_meta[wib][kk - o1];
-                        slo = m.x;
-                        own = m.y < 0;
-                        shi = own ? -m.y - 1 : m.y;
-                        sx = (double)__int_as_float(m.z);
-                        sy = (double)__int_as_float(m.w);
-                    } else {
-                        const int sc = l.l1_src[kk];
-                        slo = t.c_lo[sc];
-                        shi = t.c_hi[sc];
-                        own = sc == c;
-                        if (rel) {
-                            sx = (double)(float)(t.c_cx[sc] - ccx);
-                            sy = (double)(float)(t.c_cy[sc] - ccy);
-                        }
-                    }
-                    double tx2[kTPT], ty2[kTPT];
-                    int self[kTPT];
-                    #pragma unroll
-                    for (int k = 0; k < kTPT; ++k) {
-                        tx2[k] = tx[k] - sx;
-                        ty2[k] = ty[k] - sy;
-                        self[k] = own ? ti[k] : -1;
-                    }
-                    pair_loop4<Tr>(src, slo + split, shi, ns, tx2, ty2, self, ex, ey);
-                }
-            }
-            // sum the splits of each target: lanes tt, tt + H, ... hold its parts
-            #pragma unroll
-            for (int k = 0; k < kTPT; ++k) {
-                s_red[wib][2 * k][lane] = on ? ex[k] : 0.0;
-                s_red[wib][2 * k + 1][lane] = on ? ey[k] : 0.0;
-            }
-            __syncwarp();
-            if (split == 0) {
-                #pragma unroll
-                for (int k = 0; k < kTPT; ++k) {
-                    double sx2 = 0.0, sy2 = 0.0;
-                    for (int s2 = 0; s2 < ns; ++s2) {
-                        sx2 += s_red[wib][2 * k][s2 * H + tt];
-                        sy2 += s_red[wib][2 * k + 1][s2 * H + tt];
-                    }
-                    if (ti[k] >= 0) p2p_store(t, ti[k], sx2, sy2, fx, fy, out0, out1, velocity, u_inf, v_inf, err);
-                }
-            }
-            __syncwarp();
         }
     }
 }
@@ -1391,32 +1171,6 @@ p2p2d_tile_f32(Tree2D t, Lists2D l, const double* __restrict__ fx,
             }
         }
     }
-}
-
-// AoS (x, y, q) copy of the sorted particles for the FP64 TMA P2P (bulk
-// copies need 16-byte aligned ranges).
-__global__ void particles_aos(Tree2D t, double4* __restrict__ aos, unsigned* err) {
-    if (fatal(err)) return;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < t.n; i += gridDim.x * blockDim.x)
-        aos[i] = make_double4(t.px[i], t.py[i], t.pq[i], 0.0);
-}
-
-template <class Tr>
-cudaError_t launch_p2p_tma(const Tree2D& t, const Lists2D& l, const typename Tr::Elem* src, const Expansions2D& e,
-                           double* out0, double* out1, int velocity, double u_inf, double v_inf, unsigned* err,
-                           cudaStream_t st, int max_par) {
-    // Room for twelve full leaves: the nine neighbours at the leaf's level plus finer ones.
-    const int cap = std::min(4096, std::max(512, 12 * max_par));
-    const size_t smem = 2 * (size_t)cap * sizeof(typename Tr::Elem) + 2 * kStageCells * sizeof(StageCell) + 64;
-    static size_t smem_set = 0;
-    if (smem > smem_set) {
-        cudaError_t r = cudaFuncSetAttribute(p2p2d_tma<Tr>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (r != cudaSuccess) return r;
-        smem_set = smem;
-    }
-    p2p2d_tma<Tr><<<148 * 8, kP2PThreads, smem, st>>>(t, l, src, e.fx, e.fy, out0, out1, velocity, u_inf, v_inf, cap,
-                                                      err);
-    return cudaGetLastError();
 }
 
 }  // namespace
@@ -1793,13 +1547,6 @@ cudaError_t fmm2d_eval_combine(const Tree2D& t, const Lists2D& l, Expansions2D& 
     return cudaGetLastError();
 }
 
-cudaError_t fmm2d_p2p_out(const Tree2D& t, const Lists2D& l, const Expansions2D& e, double* out0, double* out1,
-                          int velocity, double u_inf, double v_inf, unsigned* err, cudaStream_t st, int* launches) {
-    p2p2d<<<148 * 16, kP2PThreads, 0, st>>>(t, l, e.fx, e.fy, out0, out1, velocity, u_inf, v_inf, err);
-    *launches += 1;
-    return cudaGetLastError();
-}
-
 cudaError_t fmm2d_p2p_f32(const Tree2D& t, const Lists2D& l, const Expansions2D& e, double* out0, double* out1,
                           int velocity, double u_inf, double v_inf, unsigned* err, cudaStream_t st, int* launches,
                           bool near_only, int lists) {
@@ -1816,22 +1563,23 @@ cudaError_t fmm2d_p2p_f32(const Tree2D& t, const Lists2D& l, const Expansions2D&
     return cudaGetLastError();
 }
 
-cudaError_t fmm2d_p2p_f64_tma(const Tree2D& t, const Lists2D& l, const Expansions2D& e, double4* aos, double* out0,
-                              double* out1, int velocity, double u_inf, double v_inf, unsigned* err, cudaStream_t st,
-                              int* launches, int max_par, bool near_only) {
-    particles_aos<<<148 * 8, 256, 0, st>>>(t, aos, err);
-    *launches += 2;
-    Expansions2D en = e;
-    if (near_only) en.fx = en.fy = nullptr;
-    if (max_par < 0) return launch_p2p_tma<P2PF64>(t, l, aos, en, out0, out1, velocity, u_inf, v_inf, err, st, -max_par);
-    p2p2d_warp<P2PF64><<<148 * 64 / P2PF64::kWarps, 32 * P2PF64::kWarps, 0, st>>>(
-        t, l, aos, en.fx, en.fy, out0, out1, velocity, u_inf, v_inf, err);
+cudaError_t fmm2d_p2p_f64(const Tree2D& t, const Lists2D& l, const Expansions2D& e, double* out0, double* out1,
+                          int velocity, double u_inf, double v_inf, unsigned* err, cudaStream_t st, int* launches,
+                          bool near_only, int lists) {
+    // Short blocks, as above.
+    const int grid = lists == kP2PListSpill ? 148 * 2 : 148 * 3 * 16;
+    near2d_f64<false><<<grid, 32 * kNear64Warps, 0, st>>>(t, l, near_only ? nullptr : e.fx, near_only ? nullptr : e.fy,
+                                                          out0, out1, velocity, u_inf, v_inf, lists, err);
+    *launches += 1;
     return cudaGetLastError();
 }
 
-cudaError_t fmm2d_p2p(const Tree2D& t, const Lists2D& l, const Expansions2D& e, double* ex, double* ey,
-                      unsigned* err, cudaStream_t st, int* launches) {
-    return fmm2d_p2p_out(t, l, e, ex, ey, 0, 0.0, 0.0, err, st, launches);
+cudaError_t fmm2d_p2p_potential(const Tree2D& t, const Lists2D& l, const Expansions2D& e, double* out, unsigned* err,
+                                cudaStream_t st, int* launches) {
+    near2d_f64<true><<<148 * 3 * 16, 32 * kNear64Warps, 0, st>>>(t, l, e.fx, nullptr, out, nullptr, 0, 0.0, 0.0,
+                                                                 kP2PListCsr, err);
+    *launches += 1;
+    return cudaGetLastError();
 }
 
 }  // namespace vpm

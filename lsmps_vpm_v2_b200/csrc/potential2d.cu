@@ -4,7 +4,7 @@
 //   L2L including p = 0                                                 (fmm2D.cpp:637-641)
 //   M2P   phi += Re[ a_0 log(w) - sum_{p>=1} a_p / p w^-p ]             (fmm2D.cpp:826-834)
 //   L2P   phi += Re[ sum_{p>=0} b_p w^p ]                               (fmm2D.cpp:858-866)
-//   P2P   phi += q_j log(r^2) / 2, j != i, list 1                       (fmm2D.cpp:77-122)
+//   P2P   phi += q_j log(r^2) / 2, j != i, list 1                       (fmm2D.cpp:77-122; near2d_f64)
 // All in FP64.
 #include "fmm2d.cuh"
 
@@ -84,34 +84,6 @@ eval_pot2d(Tree2D t, Lists2D l, const double2* __restrict__ a, const double2* __
     }
 }
 
-// Near-field potential over list 1 plus the far field, written in the
-// caller's order. One block per leaf, one thread per target.
-__global__ void __launch_bounds__(128)
-p2p_pot2d(Tree2D t, Lists2D l, const double* __restrict__ far, double* __restrict__ out, unsigned* err) {
-    if (fatal(err)) return;
-    const int nl = t.info->n_leaves;
-    for (int li = blockIdx.x; li < nl; li += gridDim.x) {
-        const int c = t.leaf_cells[li];
-        const int lo = t.c_lo[c], hi = t.c_hi[c];
-        const uint32_t o1 = l.l1_off[li], e1 = l.l1_off[li + 1];
-        for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-            const double x = t.px[i], y = t.py[i];
-            double phi = 0.0;
-            for (uint32_t k = o1; k < e1; ++k) {
-                const int sc = l.l1_src[k];
-                for (int j = t.c_lo[sc]; j < t.c_hi[sc]; ++j) {
-                    if (j == i) continue;
-                    const double dx = x - t.px[j], dy = y - t.py[j];
-                    phi += t.pq[j] * log(dx * dx + dy * dy) / 2.0;
-                }
-            }
-            const uint32_t orig = t.perm[i];
-            if (orig >= (uint32_t)t.n) set_err(err, ERR_INDEX);
-            else out[orig] = phi + far[i];
-        }
-    }
-}
-
 }  // namespace
 
 // Potential stages after the field's M2L: b_0, then L2L (shared), then these.
@@ -125,9 +97,9 @@ cudaError_t fmm2d_m2l_b0(const Tree2D& t, const Lists2D& l, Expansions2D& e, int
 cudaError_t fmm2d_potential_eval(const Tree2D& t, const Lists2D& l, Expansions2D& e, int P, double* out,
                                  unsigned* err, cudaStream_t st, int* launches) {
     eval_pot2d<<<148 * 16, 64, 0, st>>>(t, l, e.a, e.b, e.fx, P, err);
-    p2p_pot2d<<<148 * 16, 128, 0, st>>>(t, l, e.fx, out, err);
-    *launches += 2;
-    return cudaGetLastError();
+    *launches += 1;
+    const cudaError_t r = cudaGetLastError();
+    return r != cudaSuccess ? r : fmm2d_p2p_potential(t, l, e, out, err, st, launches);
 }
 
 }  // namespace vpm

@@ -236,7 +236,7 @@ extern "C" int vpm_fmm2d_field_device_static(const double* x, const double* y, c
         if (p.precision == VPM_PREC_MIXED || p.precision == VPM_PREC_MIXED_FP64_M2L)
             r = fmm2d_p2p_f32(t, l, xe, ex, ey, 0, 0.0, 0.0, err, st, &launches);
         else
-            r = fmm2d_p2p(t, l, xe, ex, ey, err, st, &launches);
+            r = fmm2d_p2p_f64(t, l, xe, ex, ey, 0, 0.0, 0.0, err, st, &launches);
     }
     unsigned bits = 0;
     if (r == cudaSuccess) r = cudaMemcpyAsync(&bits, err, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
