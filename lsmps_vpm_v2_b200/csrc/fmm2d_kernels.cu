@@ -638,7 +638,9 @@ constexpr int kP2PMeta = 64;   // list-1 cells staged per leaf at a time
 // FP64 operations. j == i is tested only in the steps that hold the leaf's own
 // cell (the reference's NaN of two coincident particles stays). Partial sums
 // are added over the lane groups in a fixed order.
-// 242 M pairs (778,377-particle boundary layer, caps 50/75): @NEW64@ us; the
+// 242 M pairs (778,377-particle boundary layer, caps 50/75): 249 us, 62 % of
+// the FP64 pipe's cycles (this mix of operations alone, in registers, reaches
+// 72 %: three 64-bit operands an FMA); the
 // kernel before took four targets per lane, cell by cell from global memory,
 // 379 us and a 13 us copy of the particles.
 constexpr int kNear64Warps = 4;
@@ -676,6 +678,37 @@ __device__ __forceinline__ int near_shape(int T) {
     return best;
 }
 
+// log a in FP64 without branches, so that the lane's targets run side by side
+// (CUDA's own log branches for its special cases: 94 us against 53 for the
+// near field of 120,011 particles): a = m 2^e with m in [sqrt(1/2), sqrt(2)),
+// log m = 2 atanh z, z = (m - 1) / (m + 1), by the series of atanh to z^21
+// (|z| <= 0.172: the next term is below 2^-60 of the sum; relative error at
+// most 3.3e-16 over 1e6 arguments). For normal a away from the ends of the
+// range (log_ordinary); the others take log().
+__device__ __forceinline__ bool log_ordinary(double a) {
+    return (unsigned)__double2hiint(a) - 0x01000000u < 0x7e000000u;   // 2^-1007 <= a < 2^1009, no NaN
+}
+__device__ __forceinline__ double log_series(double a) {
+    const int hi = __double2hiint(a);
+    // high word of sqrt(1/2): m >= sqrt(1/2) up to 2^-20, and e = 0 next to 1
+    const int e = (hi - 0x3fe6a09e) >> 20;
+    const double m = __hiloint2double(hi - (e << 20), __double2loint(a));
+    const double num = m - 1.0;
+    const double z = num * rcp_nr(m + 1.0);
+    const double z2 = z * z;
+    double p = fma(z2, 2.0 / 21.0, 2.0 / 19.0);
+    p = fma(p, z2, 2.0 / 17.0);
+    p = fma(p, z2, 2.0 / 15.0);
+    p = fma(p, z2, 2.0 / 13.0);
+    p = fma(p, z2, 2.0 / 11.0);
+    p = fma(p, z2, 2.0 / 9.0);
+    p = fma(p, z2, 2.0 / 7.0);
+    p = fma(p, z2, 2.0 / 5.0);
+    p = fma(p, z2, 2.0 / 3.0);
+    p = fma(p * z2, z, 2.0 * z);
+    return fma((double)e, 0.69314718055994530942, p);
+}
+
 // Staged sources s0, s0 + ns, ... below cnt onto the lane's M targets; SELF:
 // flat source self[k] is target k itself. POT: sums q log(r^2) in ex.
 template <int M, bool POT, bool SELF>
@@ -692,20 +725,30 @@ __device__ __forceinline__ void near64_pairs(const double2* xy, const double* q,
         const int sn = min(s + ns, kNear64Stage - 1);
         pn = xy[sn];
         wn = q[sn];
+        double r2[M], lg[M];
+        bool odd = false;
         #pragma unroll
         for (int k = 0; k < M; ++k) {
             const double dx = x[k] - p.x, dy = y[k] - p.y;
-            const double r2 = fma(dx, dx, dy * dy);
+            r2[k] = fma(dx, dx, dy * dy);
             if (POT) {
-                double v = w * log(r2);
-                if (SELF && s == self[k]) v = 0.0;
-                ex[k] += v;
+                lg[k] = log_series(r2[k]);
+                odd |= !log_ordinary(r2[k]);
             } else {
-                double f = w * rcp_nr(r2);
+                double f = w * rcp_nr(r2[k]);
                 if (SELF && s == self[k]) f = 0.0;
                 ex[k] = fma(f, dx, ex[k]);
                 ey[k] = fma(f, dy, ey[k]);
             }
+        }
+        if (POT) {
+            if (odd) {   // a target itself, coincident particles, or distances beyond 1e+-150
+                #pragma unroll
+                for (int k = 0; k < M; ++k)
+                    if (!log_ordinary(r2[k])) lg[k] = SELF && s == self[k] ? 0.0 : log(r2[k]);
+            }
+            #pragma unroll
+            for (int k = 0; k < M; ++k) ex[k] = fma(w, lg[k], ex[k]);
         }
     }
 }
@@ -851,7 +894,15 @@ near2d_f64(Tree2D t, Lists2D l, const double* __restrict__ fx, const double* __r
     if (fatal(err)) return;
     const int wib = threadIdx.x >> 5;
     const int nl = t.info->n_leaves;
-    for (int li = blockIdx.x * kNear64Warps + wib; li < nl; li += gridDim.x * kNear64Warps) {
+    // A tree of few leaves leaves most of the GPU's 148 x 12 warps without one:
+    // 2, 4 or 8 warps then share a leaf's targets (2,001 particles, 64 leaves:
+    // 24 -> 12 us). Splitting further than one warp per place costs more in
+    // repeated staging than it evens out (20,001 particles, about 1,024 leaves
+    // in 2 and 4 parts: the graph 133 -> 144 and 156 us).
+    int parts = 1;
+    while (parts < 8 && (long long)nl * parts * 2 <= 148 * 12) parts *= 2;
+    for (int it = blockIdx.x * kNear64Warps + wib; it < nl * parts; it += gridDim.x * kNear64Warps) {
+        const int li = it / parts, part = it - li * parts;
         const int32_t* src1;
         int n1;
         if (lists == kP2PListCsr) {
@@ -865,8 +916,10 @@ near2d_f64(Tree2D t, Lists2D l, const double* __restrict__ fx, const double* __r
             n1 = spill ? (int)(l.l1_off[li + 1] - l.l1_off[li]) : (int)cnt;
         }
         const int c = t.leaf_cells[li];
-        const int lo = t.c_lo[c], hi = t.c_hi[c];
-        for (int tb = lo; tb < hi; tb += kNear64Chunk) {
+        const int lo = t.c_lo[c], leaf_hi = t.c_hi[c];
+        const int slice = (leaf_hi - lo + parts - 1) / parts;
+        const int hi = min(leaf_hi, lo + (part + 1) * slice);
+        for (int tb = lo + part * slice; tb < hi; tb += kNear64Chunk) {
             const int T = min(kNear64Chunk, hi - tb);
             switch (near_shape(T)) {
 #define VPM_NEAR_CASE(MM)                                                                                            \
