@@ -222,6 +222,11 @@ cudaError_t fmm2d_upward(const Tree2D& t, Expansions2D& e, int P, unsigned* err,
 // the deepest level holding one) when upward_direct_ok; else fmm2d_upward.
 // Uses grid-barrier words 2 and 3 of t.gbar (zeroed before every evaluation).
 bool upward_direct_ok(int P, bool exact);
+// M2M of the active non-leaf cells of more than min_count particles, one
+// cooperative launch of at most max_grid blocks over levels *(t.gbar + 3) .. 1
+// (shift2d.cu), orders 1..18.
+cudaError_t fmm2d_m2m_big(const Tree2D& t, Expansions2D& e, int P, int min_count, int max_grid, unsigned* err,
+                          cudaStream_t st);
 // mid (may be null): recorded on st once every cell's moments except those of
 // the cells left to the M2M loop are final (at the end when there is no loop).
 cudaError_t fmm2d_upward_direct(const Tree2D& t, Expansions2D& e, int P, bool exact, unsigned* err, cudaStream_t st,
@@ -237,6 +242,7 @@ cudaError_t fmm2d_potential_eval(const Tree2D& t, const Lists2D& l, Expansions2D
 // Leaves' full local expansions straight from their ancestors' M2L parts
 // (replaces the level-by-level L2L when l2l_direct_ok: exact binomials up to
 // order P).
+constexpr int kL2LMaxP = 30;
 bool l2l_direct_ok(int P, bool exact);
 cudaError_t fmm2d_l2l_leaves(const Tree2D& t, Expansions2D& e, int P, unsigned* err, cudaStream_t st, int* launches);
 // List-2 M2L of the mixed form per parent (m2l_tc.cu, m2l_parent_tc): one
