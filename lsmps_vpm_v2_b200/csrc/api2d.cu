@@ -274,7 +274,8 @@ int Ctx::enqueue2d(const double* x, const double* y, const double* q, const uint
         VPM_CUDA_TRY(cudaEventRecord(join3, side2));
         // mixed form: the per-parent M2L of the levels below the cells left
         // to the M2M loop runs on the lists-2/4 stream as soon as the other
-        // moments are final, beside that loop; the rest follows it
+        // moments are final, beside that loop; the rest follows it (the FP64
+        // M2L split like that: no change, 334 us against 346 at 340k)
         const bool split = split_m2l && p.precision == VPM_PREC_MIXED && m2l_parent_f32_supported(p.p) &&
                            lists.l2_blk && tree.nonleaf && tree.gbar;
         VPM_CUDA_TRY(fmm2d_upward_direct(tree, ex2, p.p, p.binom == VPM_BINOM_EXACT, d_err, st, &launches,
@@ -333,8 +334,9 @@ int Ctx::enqueue2d(const double* x, const double* y, const double* q, const uint
         }
         VPM_CUDA_TRY(fmm2d_upward_direct(tree, ex2, p.p, p.binom == VPM_BINOM_EXACT, d_err, st, &launches));
         if (int r = record(4)) return r;
-        if (velocity == kModePotential) VPM_CUDA_TRY(fmm2d_m2l_only(tree, lists, ex2, p.p, d_err, st, &launches));
-        else if (int r = enqueue_m2l(p, st, &launches)) return r;
+        vpm_fmm_params pm = p;
+        if (velocity == kModePotential) pm.precision = VPM_PREC_FP64;   // the potential is FP64 in either setting
+        if (int r = enqueue_m2l(pm, st, &launches)) return r;
         if (velocity == kModePotential) VPM_CUDA_TRY(fmm2d_m2l_b0(tree, lists, ex2, p.p, d_err, st, &launches));
         if (int r = record(5)) return r;
         if (l2l_direct_ok(p.p, p.binom == VPM_BINOM_EXACT))
@@ -365,6 +367,16 @@ int Ctx::enqueue2d(const double* x, const double* y, const double* q, const uint
     return VPM_OK;
 }
 
+// Whether the FP64 M2L goes per parent cell: its blocks take 32 parents at
+// once, so a small tree leaves most of the GPU idle and is faster with a warp
+// per target cell. The line is drawn by the expected number of leaves: at cap
+// 50, 50,001 scattered particles 153 us with a warp per cell and 160 per
+// parent (captured graph), a 65,536-particle lattice 172 and 166, 120,001
+// particles 185 and 178, 340,000 particles 400 and 335.
+bool Ctx::m2l_f64_per_parent(const vpm_fmm_params& p) const {
+    return m2l_parent_f64_supported(tree, lists, p.p) && tree.n / std::max(1, std::min(p.max_src, p.max_par)) >= 1200;
+}
+
 // M2L of lists 2 and 4 for the precision setting: the mixed form per parent
 // on the FP32 pipes (orders 1..16), the tensor-core variants for
 // VPM_PREC_MIXED_TC (per parent, orders 1..16) and for the mixed orders 17..20
@@ -377,6 +389,8 @@ int Ctx::enqueue_m2l(const vpm_fmm_params& p, cudaStream_t st, int* launches) {
         VPM_CUDA_TRY(fmm2d_m2l_parent(tree, lists, ex2, p.p, tc_rows, tc_ops, d_err, st, launches));
     else if ((p.precision == VPM_PREC_MIXED || p.precision == VPM_PREC_MIXED_TC) && m2l_tc_supported(p.p))
         VPM_CUDA_TRY(fmm2d_m2l_tc(tree, lists, ex2, p.p, tc_rows, tc_ops, d_err, st, launches));
+    else if (m2l_f64_per_parent(p))
+        VPM_CUDA_TRY(fmm2d_m2l_parent_f64(tree, lists, ex2, p.p, exact, d_err, st, launches));
     else
         VPM_CUDA_TRY(fmm2d_m2l_only(tree, lists, ex2, p.p, d_err, st, launches));
     return VPM_OK;

@@ -258,6 +258,12 @@ bool m2l_parent_supported(int P);
 bool m2l_parent_f32_supported(int P);
 cudaError_t fmm2d_m2l_parent_f32(const Tree2D& t, const Lists2D& l, Expansions2D& e, int P, bool exact,
                                  unsigned* err, cudaStream_t st, int* launches, int part = 0);
+// The same in FP64 (m2l_f64.cu), the plain form's M2L of orders 1..16.
+bool m2l_parent_f64_supported(const Tree2D& t, const Lists2D& l, int P);
+cudaError_t fmm2d_m2l_parent_f64(const Tree2D& t, const Lists2D& l, Expansions2D& e, int P, bool exact,
+                                 unsigned* err, cudaStream_t st, int* launches);
+// The reference's binComb or the exact binomial (host), for the M2L coefficients.
+long long binom_m2l_host(int n, int k, bool exact);
 // List 4 (and list 2 of an irregular tree) added to b in FP64.
 cudaError_t fmm2d_m2l_list4(const Tree2D& t, const Lists2D& l, Expansions2D& e, int P, unsigned* err, cudaStream_t st,
                             int* launches);

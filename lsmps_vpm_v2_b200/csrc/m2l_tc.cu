@@ -27,8 +27,6 @@
 
 namespace vpm {
 
-namespace {
-
 // The reference's binComb (32-bit, wrapping, truncating divisions) or the
 // exact binomial coefficient, for the M2L coefficients on the host.
 long long binom_m2l_host(int n, int k, bool exact) {
@@ -44,6 +42,8 @@ long long binom_m2l_host(int n, int k, bool exact) {
     for (int i = mn; i > 1; --i) c /= i;
     return c;
 }
+
+namespace {
 
 constexpr int kTcRows = 128;
 constexpr int kTcStages = 2;
