@@ -223,8 +223,8 @@ int Ctx::enqueue2d(const double* x, const double* y, const double* q, const uint
     // gather them in tree order just before their first reader.
     const bool deferred = q_ready != nullptr && !tree_only;
     const unsigned wait_flags = capturing ? cudaEventWaitExternal : 0u;
-    VPM_CUDA_TRY(keys_sort2d(x, y, deferred ? nullptr : q, act, tree, ts, p.exp_tree_pct, d_err, st, &launches,
-                             std::min(p.max_src, p.max_par), sort_items));
+    VPM_CUDA_TRY(keys_sort2d(x, y, deferred ? nullptr : q, act, tree, ts, p.max_src, p.max_par, p.exp_tree_pct, d_err,
+                             st, &launches, true, sort_items));
     if (int r = record(1)) return r;
     VPM_CUDA_TRY(levels2d(tree, ts, p.max_src, p.max_par, d_err, st, &launches));
     if (int r = record(2)) return r;

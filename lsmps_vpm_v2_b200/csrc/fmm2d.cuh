@@ -145,6 +145,7 @@ struct TreeScratch2D {
     uint32_t* tile_cnt;     // [2][kMaxLevels2D + 1][flat_tiles] cells / leaves per tile and level, then offsets
     uint32_t* level_tot;    // [2][kMaxLevels2D + 1] cells / leaves per level
     int flat_tiles;         // tiles of kFlatTile particles
+    bool pinfo_done = false;   // pinfo of the current sort is written (keys_sort2d)
     uint32_t* coop_words;   // [kCoopSortWords] count tables of the cooperative sort (nullptr: multi-kernel sort)
     SortScratch sort;
     ScanScratch scan;
@@ -158,8 +159,9 @@ cudaError_t build_tree2d(const double* x, const double* y, const double* q, cons
 
 // The two halves of build_tree2d: bounding box, keys, sort, gather and the
 // active-count scan; then the level-by-level cell construction.
-// shallow_cap = min(max_src, max_par): lets the cooperative sort try three
-// radix passes first (see sort2d_coop); 0 always sorts the full keys.
+// max_src, max_par: the leaf caps (the cooperative sort also writes the level
+// records that depend on them, s.pinfo). shallow lets it try three radix
+// passes first (see sort2d_coop); without it the full keys are always sorted.
 // q = null sorts without the strengths: t.pq is then left for
 // gather_strengths2d, so that the strengths can still be in flight from the
 // host while the tree and the lists are built.
@@ -168,8 +170,8 @@ cudaError_t build_tree2d(const double* x, const double* y, const double* q, cons
 // the GPU in a batch take fewer, fuller blocks so that several sorts fit at
 // once).
 cudaError_t keys_sort2d(const double* x, const double* y, const double* q, const uint8_t* act, Tree2D& t,
-                        TreeScratch2D& s, double exp_pct, unsigned* err, cudaStream_t st, int* launches,
-                        int shallow_cap = 0, int items_per_block = 1024);
+                        TreeScratch2D& s, int max_src, int max_par, double exp_pct, unsigned* err, cudaStream_t st,
+                        int* launches, bool shallow = false, int items_per_block = 1024);
 // t.pq[i] = q[t.perm[i]] for i < t.n.
 cudaError_t gather_strengths2d(const Tree2D& t, const double* q, unsigned* err, cudaStream_t st, int* launches);
 cudaError_t levels2d(Tree2D& t, TreeScratch2D& s, int max_src, int max_par, unsigned* err, cudaStream_t st,

@@ -14,6 +14,8 @@
 // This file is compiled with --fmad=false: every geometric value (root box,
 // pivot, index, cell centre) is formed by separate IEEE operations in the
 // reference's order.
+#include <atomic>
+
 #include "fmm2d.cuh"
 
 namespace vpm {
@@ -156,6 +158,57 @@ __global__ void gather2d(const double* __restrict__ x, const double* __restrict_
     }
 }
 
+__device__ __forceinline__ int lcp_levels(uint64_t a, uint64_t b, int K) {
+    const uint64_t x = a ^ b;
+    if (x == 0) return K;
+    const int m = 63 - __clzll((long long)x);
+    return (2 * K - 1 - m) >> 1;
+}
+
+// Smallest m in [lo, hi] with a[m] >= target, or hi + 1 (a nondecreasing):
+// galloping from lo, then bisection.
+__device__ __forceinline__ int gallop_ge(const uint32_t* __restrict__ a, int lo, int hi, uint32_t target) {
+    if (lo > hi) return hi + 1;
+    if (__ldcg(a + lo) >= target) return lo;
+    int prev = lo, step = 1;
+    int cur = lo + 1;
+    while (cur <= hi && __ldcg(a + cur) < target) {
+        prev = cur;
+        step <<= 1;
+        cur = lo + step;
+    }
+    int L = prev + 1, R = min(cur, hi + 1);  // answer in [L, R]
+    while (L < R) {
+        const int mid = (L + R) >> 1;
+        if (__ldcg(a + mid) >= target) R = mid;
+        else L = mid + 1;
+    }
+    return L;
+}
+
+// Particle i's record for the flat build (below), lvl | (bigL + 1) << 8, from
+// the sorted keys and the active scan, read through L2 (the cooperative sort
+// has written them from other SMs).
+__device__ __forceinline__ uint32_t particle_levels(const Tree2D& t, int i, int max_src, int max_par) {
+    const int n = t.n, K = t.key_levels;
+    const uint64_t ki = __ldcg(t.key + i);
+    const int lvl = i == 0 ? 1 : lcp_levels(__ldcg(t.key + i - 1), ki, K) + 1;   // K + 1: equal keys
+    int big = -1;
+    if ((long long)i + max_par < n) big = lcp_levels(ki, __ldcg(t.key + i + max_par), K);
+    // The (max_src + 1)-th active particle from i is looked for among the next
+    // max_par particles only: further on, it shares no more digits with i
+    // than particle i + max_par does (a search beyond took 8 us more where
+    // most of 50,000 particles are inactive).
+    const uint32_t target = __ldcg(t.actscan + i) + (uint32_t)max_src + 1u;
+    const int to = (int)min((long long)n, (long long)i + max_par);
+    if (__ldcg(t.actscan + to) >= target) {
+        // as[m] - as[i] <= m - i, so m >= i + max_src + 1: start the search there
+        const int m = gallop_ge(t.actscan, (int)min((long long)to, (long long)i + max_src + 1), to, target);
+        big = max(big, lcp_levels(ki, __ldcg(t.key + m - 1), K));   // particle m-1 is that active one
+    }
+    return (uint32_t)lvl | ((uint32_t)(big + 1) << 8);
+}
+
 // ---- the sorted particle order in one cooperative launch ------------------------
 //
 // With 32-bit keys and at most kCoopSortMaxChunk particles per block, one
@@ -171,13 +224,12 @@ __global__ void gather2d(const double* __restrict__ x, const double* __restrict_
 // the multi-kernel path: the same keys, the same stable order.
 constexpr int kCoopSortThreads = 1024;
 constexpr int kCoopSortWarps = kCoopSortThreads / 32;
-constexpr int kCoopBarrierWord = 6;
+constexpr int kCoopBarrierWord = 6;   // grid-barrier words 6, 7 of Tree2D::gbar
 constexpr int kCoopRounds = 6;        // rounds of 32 items per warp loaded together
-constexpr int kCoopActRun = 16;       // sorted flags per thread in the active scan (kCoopSortMaxChunk / 1024)   // grid-barrier words 6, 7 of Tree2D::gbar
 
-// Exclusive scan over the 1024 threads of the block; *total = the block sum.
-// Every thread must call it (it holds three block barriers).
-__device__ __forceinline__ uint32_t coop_block_scan(uint32_t v, uint32_t* s_ws, uint32_t* total) {
+// Exclusive scan over the block's first 256 threads (only these call it); s8
+// is a buffer of its own for each call between two block barriers.
+__device__ __forceinline__ uint32_t scan256(uint32_t v, uint32_t* s8, uint32_t* total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t x = v;
     #pragma unroll
@@ -185,21 +237,16 @@ __device__ __forceinline__ uint32_t coop_block_scan(uint32_t v, uint32_t* s_ws, 
         const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
         if (lane >= o) x += y;
     }
-    if (lane == 31) s_ws[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = s_ws[lane];
-        #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += y;
-        }
-        s_ws[lane] = w;
+    if (lane == 31) s8[warp] = x;
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    uint32_t base = 0, tot = 0;
+    #pragma unroll
+    for (int w = 0; w < 8; ++w) {
+        const uint32_t y = s8[w];
+        if (w < warp) base += y;
+        tot += y;
     }
-    __syncthreads();
-    const uint32_t base = warp ? s_ws[warp - 1] : 0u;
-    *total = s_ws[kCoopSortWarps - 1];
-    __syncthreads();
+    *total = tot;
     return base + x - v;
 }
 
@@ -215,6 +262,7 @@ constexpr int kCwTotal = 1024 * kCoopSortGridMax;
 constexpr int kCwActTotal = kCwTotal + 256;
 constexpr int kCwFlag = kCwActTotal + 256;   // set when the shallow attempt must be redone
 static_assert(kCwFlag + 1 <= kCoopSortWords, "count tables of the cooperative sort");
+static_assert(kCoopSortMaxChunk < 1 << 16, "two counts per word, 16-bit ranks");
 
 // kb0/kb1: 32-bit key ping-pong buffers (pass 0's keys are computed into
 // kb0); vb0/vb1: index ping-pong buffers, vb1 may alias t.perm (the last
@@ -233,20 +281,60 @@ static_assert(kCwFlag + 1 <= kCoopSortWords, "count tables of the cooperative so
 // consecutive particles share a cell (shallow_cap = min(max_src, max_par)),
 // which the kernel checks after the three passes. Otherwise it sorts again
 // with all four passes.
+//
+// The flat build's per-particle records (pinfo, particle_levels) come with
+// that check: they read the same keys, and a launch of their own took 8 us.
+//
+// CLUSTER (up to 16 blocks, one thread-block cluster): the same steps with the
+// cluster's hardware barrier (0.3 to 0.6 us, against 1.3 to 2 through a word in
+// L2) and the digit counts read from the other blocks' shared memory, which
+// drops the prefix step and its barrier from every pass: eight barriers in
+// place of eleven.
+//
+// Most of a pass is latency inside the block, not the data: 26 us of 36 with
+// 1,000 particles in each of two blocks. So the rounds of a warp load, then
+// vote, then count (one chain through shared memory), rounds past the end are
+// skipped, the warps' counts are prefixed by all 1,024 threads, the digit scans
+// take one barrier of 256 threads, and nothing counts by atomics.
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The word at `p` of this block's shared memory, in block `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_ld(const uint32_t* p, int rank) {
+    uint32_t v;
+    asm volatile(
+        "{\n\t.reg .b32 ra;\n\t"
+        "mapa.shared::cluster.u32 ra, %1, %2;\n\t"
+        "ld.shared::cluster.u32 %0, [ra];\n\t}"
+        : "=r"(v)
+        : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank)
+        : "memory");
+    return v;
+}
+
+template <bool CLUSTER>
 __global__ void __launch_bounds__(kCoopSortThreads, 1)
 sort2d_coop(const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ q,
             const uint8_t* __restrict__ act, double exp_pct, int passes, int shallow_cap, Tree2D t, double* partial,
-            uint32_t* kb0, uint32_t* kb1, uint32_t* vb0, uint32_t* vb1, uint32_t* words, int chunk_cap,
-            unsigned* err) {
+            uint32_t* kb0, uint32_t* kb1, uint32_t* vb0, uint32_t* vb1, uint32_t* words, int chunk_cap, int max_src,
+            int max_par, uint32_t* __restrict__ pinfo, unsigned* err) {
     extern __shared__ __align__(16) unsigned char cs_sm[];
-    __shared__ uint32_t s_wh[kCoopSortWarps][256];   // per-warp digit counts, then warp-exclusive prefixes
+    // per-warp digit counts (last pass: active ones in the upper half), then warp-exclusive prefixes
+    __shared__ uint32_t s_wh[kCoopSortWarps][256];
     __shared__ uint32_t s_local[256];                // tile-local start of each digit
     __shared__ uint32_t s_base[256];                 // output index minus tile-local index, per digit
-    __shared__ uint32_t s_wa[256];                   // last pass: the block's active count per digit
     __shared__ uint32_t s_abase[256];                // last pass: active count before the digit's run, minus local
-    __shared__ uint32_t s_ws[32];
+    __shared__ uint32_t s_q[4][256];                 // digit counts of each quarter of the warps
+    __shared__ uint32_t s_ws[kCoopSortWarps], s_s8[4][8];
     __shared__ double s_red[4][kCoopSortWarps];
+    __shared__ double s_box[4];
     __shared__ double s_geo[3];
+    __shared__ uint32_t s_cnt[2][256];               // cluster: digit and active counts, for the other blocks
+    __shared__ uint32_t s_over;
+    auto meet = [&]() {
+        if constexpr (CLUSTER) cluster_sync_all();
+        else grid_sync_counter(t.gbar + kCoopBarrierWord, err);
+    };
     const int n = t.n;
     const int G = gridDim.x, b = blockIdx.x, tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
@@ -255,7 +343,6 @@ sort2d_coop(const double* __restrict__ x, const double* __restrict__ y, const do
         if (b == 0 && tid == 0) set_err(err, ERR_INDEX);
         return;
     }
-    unsigned* bar = t.gbar + kCoopBarrierWord;
     uint32_t* s_key = (uint32_t*)cs_sm;                  // [chunk_cap]
     uint32_t* s_val = s_key + chunk_cap;                 // [chunk_cap]
     uint16_t* s_rank = (uint16_t*)(s_val + chunk_cap);   // [chunk_cap]
@@ -266,7 +353,7 @@ sort2d_coop(const double* __restrict__ x, const double* __restrict__ y, const do
     // 1. bounding box (block partials, barrier, every block reduces all of
     //    them)
     {
-        double mnx = x[0], mxx = x[0], mny = y[0], mxy = y[0];
+        double mnx = HUGE_VAL, mxx = -HUGE_VAL, mny = HUGE_VAL, mxy = -HUGE_VAL;
         bool bad = false;
         #pragma unroll 6
         for (int i = c0 + tid; i < c1; i += kCoopSortThreads) {
@@ -285,38 +372,33 @@ sort2d_coop(const double* __restrict__ x, const double* __restrict__ y, const do
         }
         if (lane == 0) { s_red[0][warp] = mnx; s_red[1][warp] = mxx; s_red[2][warp] = mny; s_red[3][warp] = mxy; }
         __syncthreads();
-        if (tid == 0) {
-            for (int w = 1; w < kCoopSortWarps; ++w) {
-                mnx = fmin(mnx, s_red[0][w]); mxx = fmax(mxx, s_red[1][w]);
-                mny = fmin(mny, s_red[2][w]); mxy = fmax(mxy, s_red[3][w]);
-            }
-            double* pp = partial + 4 * b;
-            pp[0] = mnx; pp[1] = mxx; pp[2] = mny; pp[3] = mxy;
-        }
-        grid_sync_counter(bar, err);
-        if (warp == 0) {
-            mnx = __ldcg(partial); mxx = __ldcg(partial + 1); mny = __ldcg(partial + 2); mxy = __ldcg(partial + 3);
-            #pragma unroll 5
-            for (int bb = lane; bb < G; bb += 32) {
-                const double* pp = partial + 4 * bb;
-                mnx = fmin(mnx, __ldcg(pp)); mxx = fmax(mxx, __ldcg(pp + 1));
-                mny = fmin(mny, __ldcg(pp + 2)); mxy = fmax(mxy, __ldcg(pp + 3));
-            }
+        // warp k < 4 takes bound k: least x, greatest x, least y, greatest y
+        const double sign = warp & 1 ? -1.0 : 1.0;
+        auto least = [&](double v) {   // of v times sign
             #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                mnx = fmin(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
-                mxx = fmax(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
-                mny = fmin(mny, __shfl_xor_sync(0xffffffffu, mny, o));
-                mxy = fmax(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
-            }
-            if (lane == 0) {
-                Geom2D gg;
-                root_geometry(mnx, mxx, mny, mxy, exp_pct, t.key_levels, gg, b == 0 ? err : nullptr);
-                s_geo[0] = gg.pivx;
-                s_geo[1] = gg.pivy;
-                s_geo[2] = gg.size_k;
-                if (b == 0) *t.geom = gg;
-            }
+            for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+            return v;
+        };
+        if (warp < 4) {
+            const double v = least(sign * s_red[warp][lane]);
+            if (lane == 0) partial[4 * b + warp] = sign * v;
+        }
+        meet();
+        if (warp < 4) {
+            double v = HUGE_VAL;
+            #pragma unroll 5
+            for (int bb = lane; bb < G; bb += 32) v = fmin(v, sign * __ldcg(partial + 4 * bb + warp));
+            v = least(v);
+            if (lane == 0) s_box[warp] = sign * v;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            Geom2D gg;
+            root_geometry(s_box[0], s_box[1], s_box[2], s_box[3], exp_pct, t.key_levels, gg, b == 0 ? err : nullptr);
+            s_geo[0] = gg.pivx;
+            s_geo[1] = gg.pivy;
+            s_geo[2] = gg.size_k;
+            if (b == 0) *t.geom = gg;
         }
         __syncthreads();
     }
@@ -325,7 +407,7 @@ sort2d_coop(const double* __restrict__ x, const double* __restrict__ y, const do
 
     // 2. LSD passes of 8 bits
     const unsigned lt = (1u << lane) - 1u;
-    if (b == 0 && tid == 0) words[kCwFlag] = 0u;
+    if (!CLUSTER && b == 0 && tid == 0) words[kCwFlag] = 0u;
     const bool try_shallow = passes == 4 && shallow_cap > 0;
     for (int attempt = try_shallow ? 0 : 1; attempt < 2; ++attempt) {
     const int np = attempt == 0 ? 3 : passes;
@@ -339,110 +421,167 @@ sort2d_coop(const double* __restrict__ x, const double* __restrict__ y, const do
         const uint32_t* vin = ((np - 1 - p) & 1) ? vb1 : vb0;
         uint32_t* vout = ((np - 2 - p) & 1) ? vb1 : vb0;
         for (int i = tid; i < kCoopSortWarps * 256; i += kCoopSortThreads) (&s_wh[0][0])[i] = 0u;
-        if (tid < 256) s_wa[tid] = 0u;
         __syncthreads();
         // rank of each item among the warp's items of its digit, in index order
         for (int i0 = w0; i0 < w1; i0 += 32 * kCoopRounds) {
-            // kCoopRounds rounds of 32 items: loads first (independent), then the ranking
+            // kCoopRounds rounds of 32 items: loads first (independent, and
+            // not used before all are issued), then the ranking
             uint32_t kr[kCoopRounds], fr[kCoopRounds];
             #pragma unroll
             for (int r = 0; r < kCoopRounds; ++r) {
-                const int i = i0 + r * 32 + lane;
-                kr[r] = 0u;
-                fr[r] = 0u;
-                if (i < w1) {
-                    if (p == 0) {
-                        kr[r] = (uint32_t)particle_key(x[i], y[i], pivx, pivy, size_k, lim, err);
-                        kb0[i] = kr[r];
-                        if (last) fr[r] = act[i] ? 1u : 0u;
-                    } else {
-                        kr[r] = __ldcg(kin + i);
-                        if (last) fr[r] = __ldcg(vin + i) >> 31;
-                    }
+                kr[r] = fr[r] = 0u;
+                if (i0 + r * 32 >= w1) continue;   // warp-uniform
+                const int i = min(i0 + r * 32 + lane, w1 - 1);
+                if (p == 0) {
+                    kr[r] = (uint32_t)particle_key(x[i], y[i], pivx, pivy, size_k, lim, err);
+                    if (i0 + r * 32 + lane < w1) kb0[i] = kr[r];
+                    if (last) fr[r] = act[i];
+                } else {
+                    kr[r] = __ldcg(kin + i);
+                    if (last) fr[r] = __ldcg(vin + i) & 0x80000000u;
                 }
             }
+            // lanes holding the same digit: one ballot per digit bit; all
+            // rounds first, since only the counts below chain them
+            unsigned mm[kCoopRounds], fb[kCoopRounds];
             #pragma unroll
             for (int r = 0; r < kCoopRounds; ++r) {
-                const int i = i0 + r * 32 + lane;
-                const bool ok = i < w1;
+                mm[r] = fb[r] = 0u;
+                if (i0 + r * 32 >= w1) continue;   // warp-uniform
                 const int d = (int)((kr[r] >> shift) & 255u);
-                // lanes holding the same digit: one ballot per digit bit
-                unsigned m = __ballot_sync(0xffffffffu, ok);
+                unsigned m = __ballot_sync(0xffffffffu, i0 + r * 32 + lane < w1);
                 #pragma unroll
                 for (int bit = 0; bit < 8; ++bit) {
                     const bool bs = (d >> bit) & 1;
                     const unsigned bv = __ballot_sync(0xffffffffu, bs);
                     m &= bs ? bv : ~bv;
                 }
+                mm[r] = m;
+                if (last) fb[r] = __ballot_sync(0xffffffffu, fr[r] != 0u);
+            }
+            #pragma unroll
+            for (int r = 0; r < kCoopRounds; ++r) {
+                if (i0 + r * 32 >= w1) continue;   // warp-uniform
+                const int i = i0 + r * 32 + lane;
+                const bool ok = i < w1;
+                const int d = (int)((kr[r] >> shift) & 255u);
+                const unsigned m = mm[r];
                 uint32_t prior = 0;
                 if (ok) prior = s_wh[warp][d];
                 __syncwarp();
-                if (ok && (m & lt) == 0) s_wh[warp][d] = prior + __popc(m);
+                if (ok && (m & lt) == 0) s_wh[warp][d] = prior + __popc(m) + ((uint32_t)__popc(m & fb[r]) << 16);
                 __syncwarp();
-                if (ok) {
-                    s_rank[i - c0] = (uint16_t)(prior + __popc(m & lt));
-                    if (fr[r]) atomicAdd(&s_wa[d], 1u);
-                }
+                if (ok) s_rank[i - c0] = (uint16_t)((prior & 0xffffu) + __popc(m & lt));
             }
         }
         __syncthreads();
-        uint32_t run = 0, tot = 0;
-        if (tid < 256) {
-            for (int w = 0; w < kCoopSortWarps; ++w) {
-                const uint32_t c = s_wh[w][tid];
-                s_wh[w][tid] = run;
-                run += c;
-            }
-            words[kCwCount + (size_t)tid * kCoopSortGridMax + b] = run;
-            if (last) words[kCwActCount + (size_t)tid * kCoopSortGridMax + b] = s_wa[tid];
-        }
-        const uint32_t loc = coop_block_scan(tid < 256 ? run : 0u, s_ws, &tot);
-        if (tid < 256) s_local[tid] = loc;
-        uint32_t aloc = 0;
-        if (last) aloc = coop_block_scan(tid < 256 ? s_wa[tid] : 0u, s_ws, &tot);
-        grid_sync_counter(bar, err);
-        // prefixes over blocks, one digit column per warp: block b takes
-        // digits b + (warp + 32 m) G; lane l holds blocks 5l .. 5l+4
-        for (int d = b + warp * G; d < 256; d += kCoopSortWarps * G) {
-            #pragma unroll 1
-            for (int tb = 0; tb < (last ? 2 : 1); ++tb) {
-                const uint32_t* col = words + (tb ? kCwActCount : kCwCount) + (size_t)d * kCoopSortGridMax;
-                uint32_t v[5], sum = 0;
-                #pragma unroll
-                for (int u = 0; u < 5; ++u) {
-                    const int bb = 5 * lane + u;
-                    v[u] = bb < G ? __ldcg(col + bb) : 0u;
-                    sum += v[u];
-                }
-                uint32_t incl = sum;
-                #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t yv = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += yv;
-                }
-                uint32_t ex = incl - sum;
-                uint32_t* pre = words + (tb ? kCwActPrefix : kCwPrefix);
-                #pragma unroll
-                for (int u = 0; u < 5; ++u) {
-                    const int bb = 5 * lane + u;
-                    if (bb < G) pre[(size_t)bb * 256 + d] = ex;
-                    ex += v[u];
-                }
-                if (lane == 31) words[(tb ? kCwActTotal : kCwTotal) + d] = incl;
-            }
-        }
-        grid_sync_counter(bar, err);
+        // counts of each warp -> of the warps before it, and the block's
+        // digit counts: thread (digit, quarter of the warps)
+        uint32_t run = 0, tot = 0, aloc = 0;
         {
-            const uint32_t before = tid < 256 ? __ldcg(words + kCwPrefix + (size_t)b * 256 + tid) : 0u;
-            const uint32_t all = tid < 256 ? __ldcg(words + kCwTotal + tid) : 0u;
-            const uint32_t start = coop_block_scan(all, s_ws, &tot);
-            if (tid < 256) s_base[tid] = start + before - s_local[tid];   // modulo 2^32
+            constexpr int PER = kCoopSortWarps / 4;
+            const int d = tid & 255, qd = tid >> 8;
+            uint32_t c[PER], sum = 0;
+            #pragma unroll
+            for (int u = 0; u < PER; ++u) c[u] = s_wh[qd * PER + u][d];
+            #pragma unroll
+            for (int u = 0; u < PER; ++u) {
+                const uint32_t v = c[u];
+                c[u] = sum;
+                sum += v;
+            }
+            s_q[qd][d] = sum;
+            __syncthreads();
+            uint32_t base = 0;
+            #pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t v = s_q[k][d];
+                if (k < qd) base += v;
+                run += v;
+            }
+            #pragma unroll
+            for (int u = 0; u < PER; ++u) s_wh[qd * PER + u][d] = base + c[u];
+        }
+        if (tid < 256) {
+            const uint32_t act_run = run >> 16;   // both halves stay below 2^15
+            run &= 0xffffu;
+            if constexpr (CLUSTER) {
+                s_cnt[0][tid] = run;
+                s_cnt[1][tid] = act_run;
+            } else {
+                words[kCwCount + (size_t)tid * kCoopSortGridMax + b] = run;
+                if (last) words[kCwActCount + (size_t)tid * kCoopSortGridMax + b] = act_run;
+            }
+            s_local[tid] = scan256(run, s_s8[0], &tot);
+            if (last) aloc = scan256(act_run, s_s8[1], &tot);
+        }
+        meet();
+        uint32_t before = 0, all = 0, abefore = 0, aall = 0;
+        if constexpr (CLUSTER) {
+            if (tid < 256) {
+                #pragma unroll 8
+                for (int r = 0; r < G; ++r) {
+                    const uint32_t v = cluster_ld(&s_cnt[0][tid], r);
+                    all += v;
+                    if (r < b) before += v;
+                }
+                if (last) {
+                    #pragma unroll 8
+                    for (int r = 0; r < G; ++r) {
+                        const uint32_t v = cluster_ld(&s_cnt[1][tid], r);
+                        aall += v;
+                        if (r < b) abefore += v;
+                    }
+                }
+            }
+        } else {
+            // prefixes over blocks, one digit column per warp: block b takes
+            // digits b + (warp + 32 m) G; lane l holds blocks 5l .. 5l+4
+            for (int d = b + warp * G; d < 256; d += kCoopSortWarps * G) {
+                #pragma unroll 1
+                for (int tb = 0; tb < (last ? 2 : 1); ++tb) {
+                    const uint32_t* col = words + (tb ? kCwActCount : kCwCount) + (size_t)d * kCoopSortGridMax;
+                    uint32_t v[5], sum = 0;
+                    #pragma unroll
+                    for (int u = 0; u < 5; ++u) {
+                        const int bb = 5 * lane + u;
+                        v[u] = bb < G ? __ldcg(col + bb) : 0u;
+                        sum += v[u];
+                    }
+                    uint32_t incl = sum;
+                    #pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const uint32_t yv = __shfl_up_sync(0xffffffffu, incl, o);
+                        if (lane >= o) incl += yv;
+                    }
+                    uint32_t ex = incl - sum;
+                    uint32_t* pre = words + (tb ? kCwActPrefix : kCwPrefix);
+                    #pragma unroll
+                    for (int u = 0; u < 5; ++u) {
+                        const int bb = 5 * lane + u;
+                        if (bb < G) pre[(size_t)bb * 256 + d] = ex;
+                        ex += v[u];
+                    }
+                    if (lane == 31) words[(tb ? kCwActTotal : kCwTotal) + d] = incl;
+                }
+            }
+            meet();
+        }
+        if (tid < 256) {
+            if constexpr (!CLUSTER) {
+                before = __ldcg(words + kCwPrefix + (size_t)b * 256 + tid);
+                all = __ldcg(words + kCwTotal + tid);
+                if (last) {
+                    abefore = __ldcg(words + kCwActPrefix + (size_t)b * 256 + tid);
+                    aall = __ldcg(words + kCwActTotal + tid);
+                }
+            }
+            const uint32_t start = scan256(all, s_s8[2], &tot);
+            s_base[tid] = start + before - s_local[tid];   // modulo 2^32
             if (last) {
-                const uint32_t abefore = tid < 256 ? __ldcg(words + kCwActPrefix + (size_t)b * 256 + tid) : 0u;
-                const uint32_t aall = tid < 256 ? __ldcg(words + kCwActTotal + tid) : 0u;
                 uint32_t atot = 0;
-                const uint32_t astart = coop_block_scan(aall, s_ws, &atot);
-                if (tid < 256) s_abase[tid] = astart + abefore - aloc;
+                const uint32_t astart = scan256(aall, s_s8[3], &atot);
+                s_abase[tid] = astart + abefore - aloc;
                 if (b == 0 && tid == 0) t.actscan[n] = atot;
             }
         }
@@ -467,10 +606,11 @@ sort2d_coop(const double* __restrict__ x, const double* __restrict__ y, const do
             }
             #pragma unroll
             for (int r = 0; r < kCoopRounds; ++r) {
+                if (i0 + r * 32 >= w1) continue;   // warp-uniform
                 const int i = i0 + r * 32 + lane;
                 if (i < w1) {
                     const int d = (int)((kr[r] >> shift) & 255u);
-                    const uint32_t lp = s_local[d] + s_wh[warp][d] + s_rank[i - c0];
+                    const uint32_t lp = s_local[d] + (s_wh[warp][d] & 0xffffu) + s_rank[i - c0];
                     s_key[lp] = kr[r];
                     s_val[lp] = vr[r];
                 }
@@ -479,19 +619,21 @@ sort2d_coop(const double* __restrict__ x, const double* __restrict__ y, const do
         __syncthreads();
         const int cnt = c1 - c0;
         if (last) {
-            // active flags before each staged item (thread tid: a contiguous run), into s_rank
-            const int a0 = tid * kCoopActRun;
-            uint32_t fl[kCoopActRun], na = 0;
-            #pragma unroll
-            for (int u = 0; u < kCoopActRun; ++u) {
-                fl[u] = a0 + u < cnt ? s_val[a0 + u] >> 31 : 0u;
-                na += fl[u];
-            }
-            uint32_t ra = coop_block_scan(na, s_ws, &tot);
-            #pragma unroll
-            for (int u = 0; u < kCoopActRun; ++u) {
-                if (a0 + u < cnt) s_rank[a0 + u] = (uint16_t)ra;
-                ra += fl[u];
+            // active flags before each staged item, into s_rank: a
+            // contiguous run of whole rounds of 32 items per warp
+            const int len = (cnt + 32 * kCoopSortWarps - 1) / (32 * kCoopSortWarps) * 32, a0 = warp * len;
+            uint32_t na = 0;
+            #pragma unroll 1
+            for (int j = a0 + lane; j < a0 + len; j += 32)
+                na += __popc(__ballot_sync(0xffffffffu, j < cnt && (s_val[j] >> 31) != 0u));
+            if (lane == 0) s_ws[warp] = na;
+            __syncthreads();
+            uint32_t ra = __reduce_add_sync(0xffffffffu, lane < warp ? s_ws[lane] : 0u);
+            #pragma unroll 1
+            for (int j = a0 + lane; j < a0 + len; j += 32) {
+                const unsigned bal = __ballot_sync(0xffffffffu, j < cnt && (s_val[j] >> 31) != 0u);
+                if (j < cnt) s_rank[j] = (uint16_t)(ra + __popc(bal & lt));
+                ra += __popc(bal);
             }
             __syncthreads();
         }
@@ -519,22 +661,34 @@ sort2d_coop(const double* __restrict__ x, const double* __restrict__ y, const do
                 t.actscan[pos] = s_abase[d] + s_rank[j];
             }
         }
-        if (!last) grid_sync_counter(bar, err);
+        if (!last) meet();
     }
-    if (attempt == 1) break;
-    // is any level-(K-4) cell holding more than shallow_cap particles?
-    grid_sync_counter(bar, err);
+    meet();
+    // the flat build's records; shallow attempt: is any level-(K-4) cell
+    // holding more than shallow_cap particles?
     {
         bool over = false;
         for (int i = c0 + tid; i < c1; i += kCoopSortThreads) {
-            const int j = i + shallow_cap;
-            if (j < n && __ldcg(t.key + i) == __ldcg(t.key + j)) over = true;
+            if (attempt == 0) {
+                const int j = i + shallow_cap;
+                if (j < n && __ldcg(t.key + i) == __ldcg(t.key + j)) over = true;
+            }
+            pinfo[i] = particle_levels(t, i, max_src, max_par);
         }
-        if (__syncthreads_or(over) && tid == 0) atomicOr(&words[kCwFlag], 1u);
+        if (attempt == 1) break;
+        const int any = __syncthreads_or(over);
+        if (tid == 0) {
+            if (CLUSTER) s_over = (uint32_t)any;
+            else if (any) atomicOr(&words[kCwFlag], 1u);
+        }
     }
-    grid_sync_counter(bar, err);
-    if (__ldcg(&words[kCwFlag]) == 0u) break;
+    meet();
+    bool redo;
+    if constexpr (CLUSTER) redo = __syncthreads_or(tid < G && cluster_ld(&s_over, tid) != 0u) != 0;
+    else redo = __ldcg(&words[kCwFlag]) != 0u;
+    if (!redo) break;
     }
+    if constexpr (CLUSTER) cluster_sync_all();   // no block leaves while another reads its shared memory
 }
 
 // ---- flat build: every level at once ------------------------------------------
@@ -563,34 +717,6 @@ sort2d_coop(const double* __restrict__ x, const double* __restrict__ y, const do
 // Kernels: flat_bigl (lvl, bigL), flat_cells (cell levels, tile counts),
 // flat_scan (scanned counts, level totals), flat_emit (cell records, parents,
 // first children), flat_link (range ends, counts, activity, child masks).
-
-__device__ __forceinline__ int lcp_levels(uint64_t a, uint64_t b, int K) {
-    const uint64_t x = a ^ b;
-    if (x == 0) return K;
-    const int m = 63 - __clzll((long long)x);
-    return (2 * K - 1 - m) >> 1;
-}
-
-// Smallest m in [lo, hi] with a[m] >= target, or hi + 1 (a nondecreasing):
-// galloping from lo, then bisection.
-__device__ __forceinline__ int gallop_ge(const uint32_t* __restrict__ a, int lo, int hi, uint32_t target) {
-    if (lo > hi) return hi + 1;
-    if (a[lo] >= target) return lo;
-    int prev = lo, step = 1;
-    int cur = lo + 1;
-    while (cur <= hi && a[cur] < target) {
-        prev = cur;
-        step <<= 1;
-        cur = lo + step;
-    }
-    int L = prev + 1, R = min(cur, hi + 1);  // answer in [L, R]
-    while (L < R) {
-        const int mid = (L + R) >> 1;
-        if (a[mid] >= target) R = mid;
-        else L = mid + 1;
-    }
-    return L;
-}
 
 // First j <= i with the same key prefix (>> sh) as particle i, with the whole
 // warp on one query (i and sh the same in every lane): 32 probes per round,
@@ -629,25 +755,11 @@ __device__ __forceinline__ uint32_t compact2(uint64_t x) {
     return (uint32_t)x;
 }
 
-// pinfo[i] = lvl | (bigL + 1) << 8
+// The multi-kernel sort's flat_bigl (the cooperative one does it itself).
 __global__ void __launch_bounds__(kFlatTile)
 flat_bigl(Tree2D t, int max_src, int max_par, uint32_t* __restrict__ pinfo, unsigned* err) {
-    const int n = t.n, K = t.key_levels;
-    const uint64_t* __restrict__ key = t.key;
-    const uint32_t* __restrict__ as = t.actscan;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint64_t ki = key[i];
-        const int lvl = i == 0 ? 1 : lcp_levels(key[i - 1], ki, K) + 1;   // K + 1: equal keys
-        int big = -1;
-        if (i + max_par < n) big = lcp_levels(ki, key[i + max_par], K);
-        const uint32_t target = as[i] + (uint32_t)max_src + 1u;
-        if (as[n] >= target) {
-            // as[m] - as[i] <= m - i, so m >= i + max_src + 1: start the search there
-            const int m = gallop_ge(as, min(n, i + max_src + 1), n, target);  // particle m-1 is that active one
-            big = max(big, lcp_levels(ki, key[m - 1], K));
-        }
-        pinfo[i] = (uint32_t)lvl | ((uint32_t)(big + 1) << 8);
-    }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < t.n; i += gridDim.x * blockDim.x)
+        pinfo[i] = particle_levels(t, i, max_src, max_par);
 }
 
 // The cell levels of every particle (pinfo bits 16..23 first, 24..31 last; 0 =
@@ -1024,13 +1136,13 @@ bool coop_sort_shape(int n, int items, int* grid, int* chunk) {
     const int c = ceil_div(n, g);
     if (c > kCoopSortMaxChunk) return false;
     if (smem_set == 0) {
-        if (cudaFuncSetAttribute(sort2d_coop, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (cudaFuncSetAttribute(sort2d_coop<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  kCoopSortMaxChunk * 10) != cudaSuccess)
             return false;
         smem_set = 1;
     }
     int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sort2d_coop, kCoopSortThreads, (size_t)c * 10) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sort2d_coop<false>, kCoopSortThreads, (size_t)c * 10) !=
             cudaSuccess ||
         occ < 1)
         return false;
@@ -1039,10 +1151,53 @@ bool coop_sort_shape(int n, int items, int* grid, int* chunk) {
     return true;
 }
 
+// Blocks of the cluster sort for n particles, about kClusterItems each, or 0
+// when the grid version takes the call: more particles than 16 blocks sort in
+// less time than the grid's SMs, a solve that shares the GPU (items_per_block
+// above 1024: its sorts already overlap others' work), or a device that cannot
+// place the cluster.
+// Captured mixed evaluation, cluster against grid: 2,001 particles 101 against
+// 121 us, 20,001 117 against 121, 32,001 120 against 123, 50,001 148 against 141.
+constexpr int kClusterItems = 1024;
+constexpr int kClusterMaxBlocks = 16;
+constexpr int kClusterMaxN = 32768;
+
+int cluster_sort_blocks(int n, int items_per_block) {
+    if (n > kClusterMaxN || items_per_block > kClusterItems) return 0;
+    int g = 1;
+    while (g < kClusterMaxBlocks && g * kClusterItems < n) g *= 2;
+    static std::atomic<int> state[64];   // per device: 0 not asked, 1 usable, -1 not
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    if (state[dev] == 0) {
+        int clusters = 0;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kClusterMaxBlocks);
+        cfg.blockDim = dim3(kCoopSortThreads);
+        cfg.dynamicSmemBytes = (size_t)ceil_div(kClusterMaxN, kClusterMaxBlocks) * 10;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = kClusterMaxBlocks;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        const bool ok =
+            cudaFuncSetAttribute(sort2d_coop<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)cfg.dynamicSmemBytes) == cudaSuccess &&
+            cudaFuncSetAttribute(sort2d_coop<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&clusters, sort2d_coop<true>, &cfg) == cudaSuccess && clusters > 0;
+        if (!ok) (void)cudaGetLastError();
+        state[dev] = ok ? 1 : -1;
+    }
+    return state[dev] > 0 ? g : 0;
+}
+
 cudaError_t keys_sort2d(const double* x, const double* y, const double* q, const uint8_t* act, Tree2D& t,
-                        TreeScratch2D& s, double exp_pct, unsigned* err, cudaStream_t st, int* launches,
-                        int shallow_cap, int items_per_block) {
+                        TreeScratch2D& s, int max_src, int max_par, double exp_pct, unsigned* err, cudaStream_t st,
+                        int* launches, bool shallow, int items_per_block) {
     const int n = t.n;
+    const int shallow_cap = shallow ? std::min(max_src, max_par) : 0;
+    s.pinfo_done = false;
     const int K = t.key_levels;
     const int gridN = std::max(1, std::min(148 * 8, ceil_div(n, 256)));
     unsigned* done = s.lvl_ticket + kMaxLevels2D + 1;
@@ -1051,7 +1206,12 @@ cudaError_t keys_sort2d(const double* x, const double* y, const double* q, const
     if (e != cudaSuccess) return e;
     *launches += 1;
     int coop_grid = 0, coop_chunk = 0;
-    if (2 * K <= 32 && s.coop_words && coop_sort_shape(n, items_per_block, &coop_grid, &coop_chunk)) {
+    const int cluster = 2 * K <= 32 && s.coop_words ? cluster_sort_blocks(n, items_per_block) : 0;
+    if (cluster) {
+        coop_grid = cluster;
+        coop_chunk = ceil_div(n, cluster);
+    }
+    if (cluster || (2 * K <= 32 && s.coop_words && coop_sort_shape(n, items_per_block, &coop_grid, &coop_chunk))) {
         uint32_t* k32 = reinterpret_cast<uint32_t*>(s.key_alt);
         const size_t smem = (size_t)coop_chunk * 10;
         cudaLaunchConfig_t cfg = {};
@@ -1060,14 +1220,21 @@ cudaError_t keys_sort2d(const double* x, const double* y, const double* q, const
         cfg.dynamicSmemBytes = smem;
         cfg.stream = st;
         cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeCooperative;
-        attr[0].val.cooperative = 1;
+        if (cluster) {
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = cluster;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        } else {
+            attr[0].id = cudaLaunchAttributeCooperative;
+            attr[0].val.cooperative = 1;
+        }
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, sort2d_coop, x, y, q, act, exp_pct, (2 * K + 7) / 8, shallow_cap, t,
-                               s.bbox_partial,
-                               k32, k32 + n, s.val_alt, t.perm, s.coop_words, coop_chunk,
+        e = cudaLaunchKernelEx(&cfg, cluster ? sort2d_coop<true> : sort2d_coop<false>, x, y, q, act, exp_pct,
+                               (2 * K + 7) / 8, shallow_cap, t, s.bbox_partial,
+                               k32, k32 + n, s.val_alt, t.perm, s.coop_words, coop_chunk, max_src, max_par, s.pinfo,
                                err);
+        s.pinfo_done = true;
         if (e != cudaSuccess) return e;
         *launches += 1;
         return cudaGetLastError();
@@ -1128,14 +1295,17 @@ cudaError_t levels2d_flat(Tree2D& t, TreeScratch2D& s, int max_src, int max_par,
     const int tiles = ceil_div(n, kFlatTile);
     if (tiles > s.flat_tiles) return cudaErrorInvalidValue;
     const int grid = std::max(1, std::min(tiles, 148 * 8));
-    flat_bigl<<<grid, kFlatTile, 0, st>>>(t, max_src, max_par, s.pinfo, err);
+    if (!s.pinfo_done) {
+        flat_bigl<<<grid, kFlatTile, 0, st>>>(t, max_src, max_par, s.pinfo, err);
+        *launches += 1;
+    }
     flat_cells<<<grid, kFlatTile, 0, st>>>(t, s.pinfo, s.tile_cnt, tiles, err);
     // lvl_ticket[0]: zeroed with the other tickets before the sort
     flat_scan<<<2 * (t.key_levels + 1), 1024, 0, st>>>(t, s.tile_cnt, tiles, s.level_tot, s.lvl_ticket, err);
     flat_emit<<<grid, kFlatTile, 0, st>>>(t, s.pinfo, s.tile_cnt, tiles, max_par, err);
     const int gc = std::max(1, std::min(148 * 8, ceil_div(t.cap_cells, 256)));
     flat_link<<<gc, 256, 0, st>>>(t, max_par, err);
-    *launches += 5;
+    *launches += 4;
     return cudaGetLastError();
 }
 
@@ -1148,7 +1318,7 @@ cudaError_t levels2d(Tree2D& t, TreeScratch2D& s, int max_src, int max_par, unsi
 cudaError_t build_tree2d(const double* x, const double* y, const double* q, const uint8_t* act, Tree2D& t,
                          TreeScratch2D& s, int max_src, int max_par, double exp_pct, unsigned* err, cudaStream_t st,
                          int* launches) {
-    cudaError_t e = keys_sort2d(x, y, q, act, t, s, exp_pct, err, st, launches, std::min(max_src, max_par));
+    cudaError_t e = keys_sort2d(x, y, q, act, t, s, max_src, max_par, exp_pct, err, st, launches, true);
     if (e != cudaSuccess) return e;
     return levels2d(t, s, max_src, max_par, err, st, launches);
 }
