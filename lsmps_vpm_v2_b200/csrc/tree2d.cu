@@ -197,8 +197,8 @@ __device__ __forceinline__ uint32_t particle_levels(const Tree2D& t, int i, int 
     if ((long long)i + max_par < n) big = lcp_levels(ki, __ldcg(t.key + i + max_par), K);
     // The (max_src + 1)-th active particle from i is looked for among the next
     // max_par particles only: further on, it shares no more digits with i
-    // than particle i + max_par does (a search beyond took 8 us more where
-    // most of 50,000 particles are inactive).
+    // than particle i + max_par does (the sort of 50,000 particles, many inactive,
+    // took 56 us with a search beyond, 52 without).
     const uint32_t target = __ldcg(t.actscan + i) + (uint32_t)max_src + 1u;
     const int to = (int)min((long long)n, (long long)i + max_par);
     if (__ldcg(t.actscan + to) >= target) {
@@ -1156,8 +1156,8 @@ bool coop_sort_shape(int n, int items, int* grid, int* chunk) {
 // less time than the grid's SMs, a solve that shares the GPU (items_per_block
 // above 1024: its sorts already overlap others' work), or a device that cannot
 // place the cluster.
-// Captured mixed evaluation, cluster against grid: 2,001 particles 101 against
-// 121 us, 20,001 117 against 121, 32,001 120 against 123, 50,001 148 against 141.
+// Captured mixed evaluation, cluster against grid: 2,001 particles 98 against
+// 115 us, 20,001 121 against 124, 32,001 127 against 128, 50,001 166 against 155.
 constexpr int kClusterItems = 1024;
 constexpr int kClusterMaxBlocks = 16;
 constexpr int kClusterMaxN = 32768;
