@@ -98,7 +98,8 @@ int Ctx::reserve2d(int n, int cap_cells, int P, long long cap_l1, long long cap_
     size_t o_l4 = L.take<int32_t>(C * kList4Cap), o_l4n = L.take<uint8_t>(C);
     size_t o_l1c = L.take<uint32_t>(C), o_l1o = L.take<uint32_t>(C + 1), o_l1s = L.take<int32_t>(cap_l1);
     size_t o_l3c = L.take<uint32_t>(C), o_l3o = L.take<uint32_t>(C + 1), o_l3s = L.take<int32_t>(cap_l3);
-    size_t o_l1slot = L.take<int32_t>(C * kListSlot1), o_l3slot = L.take<int32_t>(C * kListSlot3);
+    size_t o_l1slot = L.take<int32_t>(C * kListSlot1), o_l3slot = L.take<int32_t>(C * kListSlot3),
+           o_csr = L.take<uint64_t>(csr_words(cap_cells));
     size_t o_a = L.take<double2>(C * (P + 1)), o_b = L.take<double2>(C * (P + 1)), o_cnt = L.take<unsigned>(C);
     size_t o_fx = L.take<double>(n), o_fy = L.take<double>(n);
     size_t o_nx = L.take<double>(n), o_ny = L.take<double>(n);
@@ -152,6 +153,7 @@ int Ctx::reserve2d(int n, int cap_cells, int P, long long cap_l1, long long cap_
     lists.l1_cnt = (uint32_t*)P_(o_l1c); lists.l1_off = (uint32_t*)P_(o_l1o); lists.l1_src = (int32_t*)P_(o_l1s);
     lists.l3_cnt = (uint32_t*)P_(o_l3c); lists.l3_off = (uint32_t*)P_(o_l3o); lists.l3_src = (int32_t*)P_(o_l3s);
     lists.l1_slot = (int32_t*)P_(o_l1slot); lists.l3_slot = (int32_t*)P_(o_l3slot);
+    lists.csr_status = (uint64_t*)P_(o_csr);
     lists.cap_leaves = cap_cells;
     lists.cap_l1 = cap_l1;
     lists.cap_l3 = cap_l3;

@@ -113,6 +113,7 @@ struct Lists2D {
     int32_t* l2_blk;
     int32_t* l1_slot;    // [cap_leaves][kListSlot1] one-pass staging of list 1 (nullptr: two passes)
     int32_t* l3_slot;    // [cap_leaves][kListSlot3]
+    uint64_t* csr_status;   // [csr_words(cap_leaves)] tile words and ticket of the CSR (with the slots)
     int cap_leaves;
     long long cap_l1, cap_l3;
 };
@@ -134,6 +135,10 @@ constexpr int kBarrierWordsAt = kMaxLevels2D + 2;
 constexpr int kCoopSortGridMax = 160;
 constexpr int kCoopSortMaxChunk = 16384;
 constexpr int kCoopSortWords = 1024 * kCoopSortGridMax + 544;
+
+// Leaves per tile of the CSR of lists 1/3 in one launch, and the words its tiles' look-back takes.
+constexpr int kCsrTile = 64;
+inline int csr_words(long long cap_leaves) { return ceil_div(cap_leaves, kCsrTile) + 1; }
 
 struct TreeScratch2D {
     double* bbox_partial;   // [kBBoxBlocks * 4]

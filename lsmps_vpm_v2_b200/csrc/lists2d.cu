@@ -352,17 +352,21 @@ __device__ void int_list_warp(const TreeView& v, int c, double eps, int mode, ui
 
 // Counts and the first kListSlot1 / kListSlot3 entries of lists 1 and 3 of
 // every leaf into fixed slots, in one pass; one warp per leaf.
-__global__ void __launch_bounds__(128) int_list_slots(Tree2D t, double eps, Lists2D l, unsigned* err) {
-    __shared__ WarpQueue s_q[4];
-    if (fatal(err)) return;
+// Block `b` of `nb`.
+__device__ __forceinline__ void int_slots_body(const Tree2D& t, double eps, const Lists2D& l, WarpQueue* s_q, int b,
+                                               int nb, unsigned* err) {
     TreeView v(t);
     const int nl = t.info->n_leaves;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    for (int i = nl + blockIdx.x * blockDim.x + threadIdx.x; i < l.cap_leaves; i += gridDim.x * blockDim.x) {
+    // the scans run over all cap_leaves counts
+    for (int i = nl + b * blockDim.x + threadIdx.x; i < l.cap_leaves; i += nb * blockDim.x) {
         l.l1_cnt[i] = 0;
         l.l3_cnt[i] = 0;
     }
-    for (int i = blockIdx.x * 4 + wib; i < nl; i += gridDim.x * 4) {
+    // the fused CSR's look-back words and ticket start at zero
+    for (int i = b * blockDim.x + threadIdx.x; i < ceil_div(nl, kCsrTile) + 1; i += nb * blockDim.x)
+        l.csr_status[i] = 0ull;
+    for (int i = b * 4 + wib; i < nl; i += nb * 4) {
         uint32_t n1, n3;
         int_list_warp(v, t.leaf_cells[i], eps, 2, &n1, &n3, l.l1_slot + (size_t)i * kListSlot1,
                       l.l3_slot + (size_t)i * kListSlot3, kListSlot1, kListSlot3, 0, 0, s_q[wib], err);
@@ -372,6 +376,12 @@ __global__ void __launch_bounds__(128) int_list_slots(Tree2D t, double eps, List
         }
         __syncwarp();
     }
+}
+
+__global__ void __launch_bounds__(128) int_list_slots(Tree2D t, double eps, Lists2D l, unsigned* err) {
+    __shared__ WarpQueue s_q[4];
+    if (fatal(err)) return;
+    int_slots_body(t, eps, l, s_q, blockIdx.x, gridDim.x, err);
 }
 
 // Slots to CSR, one warp per leaf; a leaf whose list outgrew its slots is
@@ -407,6 +417,107 @@ __global__ void int_list_overflow(Tree2D t, double eps, Lists2D l, unsigned* err
                  l.l3_off[i], err);
     }
 }
+
+// Offsets of lists 1 and 3 of every leaf, their entries from the slots into
+// the CSR, the leaves that outgrew their slots and the totals, in one launch
+// (five kernels before, of 31 us together at 22,927 leaves and 23 us at 64):
+// a tile of kCsrTile leaves per block, the two counts of a leaf side by side
+// in one word (capacities up to 2^31 - 1, build_lists2d), tile prefixes by look-back (tiles take their number from a
+// ticket, so a tile waits only on tiles that already run; bounded).
+constexpr uint64_t kCsrA = 1ull << 62, kCsrP = 2ull << 62, kCsrMask = (1ull << 62) - 1;
+constexpr uint64_t kCsrLow = (1ull << 31) - 1;
+constexpr int kCsrThreads = 256;
+constexpr int kCsrPerWarp = kCsrTile / (kCsrThreads / 32);   // leaves a warp copies, loads before stores
+
+__global__ void __launch_bounds__(kCsrThreads) int_list_csr(Tree2D t, double eps, Lists2D l, unsigned* err) {
+    __shared__ uint64_t s_w[kCsrThreads / 32], s_base;
+    __shared__ uint32_t s_n1[kCsrTile], s_n3[kCsrTile], s_o1[kCsrTile], s_o3[kCsrTile];
+    __shared__ int s_tile;
+    if (block_fatal(err)) return;
+    TreeView v(t);
+    const int nl = t.info->n_leaves, tiles = ceil_div(nl, kCsrTile);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t* status = l.csr_status + 1;
+    for (;;) {
+        __syncthreads();   // the last tile's shared words are read
+        if (threadIdx.x == 0) s_tile = (int)atomicAdd(reinterpret_cast<unsigned long long*>(l.csr_status), 1ull);
+        __syncthreads();
+        const int tile = s_tile;
+        if (tile >= tiles) return;   // block-uniform
+        const int i = tile * kCsrTile + threadIdx.x;
+        const bool mine = threadIdx.x < kCsrTile && i < nl;
+        const uint32_t n1 = mine ? l.l1_cnt[i] : 0u, n3 = mine ? l.l3_cnt[i] : 0u;
+        const uint64_t w = (uint64_t)n1 | ((uint64_t)n3 << 31);
+        uint64_t x = w;
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) s_w[warp] = x;
+        __syncthreads();
+        uint64_t before = 0, all = 0;
+        #pragma unroll
+        for (int k = 0; k < kCsrThreads / 32; ++k) {
+            if (k < warp) before += s_w[k];
+            all += s_w[k];
+        }
+        if (warp == 0) {
+            if (lane == 0) st_relaxed64(&status[tile], (tile == 0 ? kCsrP : kCsrA) | all);
+            const uint64_t base = tile == 0 ? 0ull : warp_lookback<kCsrP, kCsrMask>(status, tile, err);
+            if (lane == 0) {
+                if (tile > 0) st_relaxed64(&status[tile], kCsrP | (base + all));
+                s_base = base;
+            }
+        }
+        __syncthreads();
+        const uint64_t at = s_base + before + x - w;
+        const uint32_t o1 = (uint32_t)(at & kCsrLow), o3 = (uint32_t)(at >> 31);
+        if (threadIdx.x < kCsrTile) {
+            s_n1[threadIdx.x] = n1;
+            s_n3[threadIdx.x] = n3;
+            s_o1[threadIdx.x] = o1;
+            s_o3[threadIdx.x] = o3;
+        }
+        if (mine) {
+            l.l1_off[i] = o1;
+            l.l3_off[i] = o3;
+            if (i == nl - 1) {
+                l.l1_off[nl] = o1 + n1;
+                l.l3_off[nl] = o3 + n3;
+                t.info->list1_len = o1 + n1;
+                t.info->list3_len = o3 + n3;
+            }
+            // a list that outgrew its slots (or the CSR, which sets the error) is made again
+            const bool big1 = n1 > kListSlot1 || (long long)o1 + n1 > l.cap_l1;
+            const bool big3 = n3 > kListSlot3 || (long long)o3 + n3 > l.cap_l3;
+            if (big1 || big3) {
+                uint32_t m1, m3;
+                int_list(v, t.leaf_cells[i], eps, 1, &m1, &m3, l.l1_src, l.l3_src, l.cap_l1, l.cap_l3, o1, o3, err);
+            }
+        }
+        __syncthreads();
+        int32_t v1[kCsrPerWarp], v3[kCsrPerWarp];
+        bool p1[kCsrPerWarp], p3[kCsrPerWarp];
+        #pragma unroll
+        for (int k = 0; k < kCsrPerWarp; ++k) {
+            const int j = warp * kCsrPerWarp + k;   // leaves past the end have counts of zero
+            const size_t leaf = (size_t)tile * kCsrTile + j;
+            const uint32_t m1 = s_n1[j], m3 = s_n3[j];
+            p1[k] = m1 <= kListSlot1 && (long long)s_o1[j] + m1 <= l.cap_l1 && lane < m1;
+            p3[k] = m3 <= kListSlot3 && (long long)s_o3[j] + m3 <= l.cap_l3 && lane < m3;
+            if (p1[k]) v1[k] = l.l1_slot[leaf * kListSlot1 + lane];
+            if (p3[k]) v3[k] = l.l3_slot[leaf * kListSlot3 + lane];
+        }
+        #pragma unroll
+        for (int k = 0; k < kCsrPerWarp; ++k) {
+            const int j = warp * kCsrPerWarp + k;
+            if (p1[k]) l.l1_src[s_o1[j] + lane] = v1[k];
+            if (p3[k]) l.l3_src[s_o3[j] + lane] = v3[k];
+        }
+    }
+}
+static_assert(kListSlot1 <= 32 && kListSlot3 <= 32, "one lane per slot");
 
 __global__ void int_list_kernel(Tree2D t, double eps, int mode, Lists2D l, unsigned* err) {
     if (fatal(err)) return;
@@ -533,22 +644,37 @@ __device__ void ext_list_warp(const TreeView& v, int c, double eps, int32_t* l2,
     __syncwarp();
 }
 
-__global__ void __launch_bounds__(128) ext_list_kernel(Tree2D t, double eps, Lists2D l, unsigned* err) {
-    __shared__ int s_e[4][8];
-    if (fatal(err)) return;
+// Block `b` of `nb`.
+__device__ __forceinline__ void ext_list_body(const Tree2D& t, double eps, const Lists2D& l, int (*s_e)[8], int b,
+                                              int nb, unsigned* err) {
     TreeView v(t);
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int wib = threadIdx.x >> 5;
     const int c0 = t.info->level_start[2], c1 = t.info->n_cells;
-    const int warps = gridDim.x * 4;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < t.cap_cells; i += gridDim.x * blockDim.x)
+    for (int i = b * blockDim.x + threadIdx.x; i < t.cap_cells; i += nb * blockDim.x)
         if (i < c0 || i >= c1) {
             l.l2_n[i] = 0;
             l.l4_n[i] = 0;
         }
-    for (int i = c0 + blockIdx.x * 4 + wib; i < c1; i += warps)
+    for (int i = c0 + b * 4 + wib; i < c1; i += nb * 4)
         ext_list_warp(v, i, eps, l.l2_src + (size_t)i * kList2Cap, l.l2_slot + (size_t)i * kList2Cap, &l.l2_n[i],
                       l.l4_src + (size_t)i * kList4Cap, &l.l4_n[i], l.l2_blk, s_e[wib], err);
-    (void)lane;
+}
+
+__global__ void __launch_bounds__(128) ext_list_kernel(Tree2D t, double eps, Lists2D l, unsigned* err) {
+    __shared__ int s_e[4][8];
+    if (fatal(err)) return;
+    ext_list_body(t, eps, l, s_e, blockIdx.x, gridDim.x, err);
+}
+
+// Lists 2/4 and the slots of lists 1/3 side by side (neither reads the
+// other), even blocks the one, odd blocks the other: for launches in order on
+// one stream, where each would wait for the last block of the other.
+__global__ void __launch_bounds__(128) lists_kernel(Tree2D t, double eps, Lists2D l, unsigned* err) {
+    __shared__ WarpQueue s_q[4];
+    __shared__ int s_e[4][8];
+    if (fatal(err)) return;
+    if (blockIdx.x & 1) int_slots_body(t, eps, l, s_q, blockIdx.x >> 1, gridDim.x >> 1, err);
+    else ext_list_body(t, eps, l, s_e, blockIdx.x >> 1, gridDim.x >> 1, err);
 }
 
 // Interaction totals for the statistics.
@@ -573,6 +699,22 @@ cudaError_t build_ext_lists2d(const Tree2D& t, Lists2D& l, double eps, unsigned*
 
 cudaError_t build_lists2d(const Tree2D& t, Lists2D& l, ScanScratch& scan, double eps, unsigned* err,
                           cudaStream_t st, int* launches) {
+    // One stream in order: two launches in place of seven (53 -> 21 us with
+    // 64 leaves, 96 -> 62 with 22,927). The captured evaluation, whose
+    // lists run on three streams, keeps the separate kernels: with int_list_csr
+    // there it took 158 us against 154 (65,536 particles) and 518 against 512
+    // (778,377), each kernel alone being no slower; the reason was not found.
+    // int_list_csr packs two 31-bit totals in a word.
+    if (int_lists_slotted(l) && l.csr_status && l.cap_l1 <= (long long)kCsrLow && l.cap_l3 <= (long long)kCsrLow) {
+        lists_kernel<<<148 * 32, 128, 0, st>>>(t, eps, l, err);
+        *launches += 1;
+        cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        int_list_csr<<<std::max(1, std::min(148 * 4, ceil_div(l.cap_leaves, kCsrTile))), kCsrThreads, 0, st>>>(t, eps, l,
+                                                                                                              err);
+        *launches += 1;
+        return cudaGetLastError();
+    }
     cudaError_t e = build_ext_lists2d(t, l, eps, err, st, launches);
     if (e != cudaSuccess) return e;
     return build_int_lists2d(t, l, scan, eps, err, st, launches);
