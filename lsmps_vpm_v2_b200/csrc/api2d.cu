@@ -230,7 +230,7 @@ int Ctx::enqueue2d(const double* x, const double* y, const double* q, const uint
     if (int r = record(1)) return r;
     VPM_CUDA_TRY(levels2d(tree, ts, p.max_src, p.max_par, d_err, st, &launches));
     if (int r = record(2)) return r;
-    if (capturing && !split_capture && !tree_only && velocity != kModePotential) {
+    if (capturing && branches && !split_capture && !tree_only && velocity != kModePotential) {
         // One captured graph: the near field (lists 1/3, P2P) runs on the side
         // stream concurrently with lists 2/4 and the far field (P2M, M2M, M2L,
         // L2L); M2P follows lists 2/4 on the third stream once the upward pass
@@ -278,7 +278,7 @@ int Ctx::enqueue2d(const double* x, const double* y, const double* q, const uint
         // to the M2M loop runs on the lists-2/4 stream as soon as the other
         // moments are final, beside that loop; the rest follows it (the FP64
         // M2L split like that: no change, 334 us against 346 at 340k)
-        const bool split = split_m2l && p.precision == VPM_PREC_MIXED && m2l_parent_f32_supported(p.p) &&
+        const bool split = p.precision == VPM_PREC_MIXED && m2l_parent_f32_supported(p.p) &&
                            lists.l2_blk && tree.nonleaf && tree.gbar;
         VPM_CUDA_TRY(fmm2d_upward_direct(tree, ex2, p.p, p.binom == VPM_BINOM_EXACT, d_err, st, &launches,
                                          split ? ev_small : nullptr));

@@ -133,10 +133,14 @@ struct Ctx {
     // particle lattice spreads over 64 SMs: 0.183 -> 0.179 ms against 2048),
     // more in the sub-contexts of a batch, whose solves share the GPU
     int sort_items = 1024;
-    // mixed form: the M2L of the levels below the large cells beside their M2M
-    // loop (one graph per solve); off in the sub-contexts of a batch, whose
-    // small solves share the GPU and gain nothing from the extra launch
-    bool split_m2l = true;
+    // A captured evaluation forks onto the side streams. Off in the
+    // sub-contexts of a batch: the other solves fill the GPU there, and a solve
+    // in order has half the launches, no events and no separate near-field and
+    // spill passes (64 solves of 4,096 to 400,000, mixed: 4.32 -> 3.90 ms; 16 of
+    // 1,000 to 20,000, FP64: 0.655 -> 0.510; 4 of 100,000 to 400,000: 0.571 ->
+    // 0.563; with the branches kept and the one-launch CSR of lists 1/3: 4.02,
+    // 0.543, 0.558).
+    bool branches = true;
 
     // batched solves (batch2d.cu)
     std::vector<Ctx*> subs;
