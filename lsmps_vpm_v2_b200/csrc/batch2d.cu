@@ -63,7 +63,8 @@ int Ctx::prepare_batch(int ns, const int64_t* offs, const vpm_fmm_params& p, int
             return fail(r, "sub-context: " + m);
         }
         // 8192 particles per sort block: a batch's sorts run side by side
-        // (64 uneven solves: 5.11 -> 4.54 ms against 2048)
+        // (64 uneven solves: 3.90 ms, against 4.45 with 2048 and 4.08 with 4096; four
+        // large ones: 0.56, against 0.64 with 16384)
         c->sort_items = 8192;
         c->branches = false;
         subs.push_back(c);
