@@ -99,8 +99,9 @@ constexpr int kLeafShiftWarps = 2;   // few leaves per SM: small blocks spread t
 
 template <int P>
 __global__ void __launch_bounds__(32 * kLeafShiftWarps)
-l2l_leaves2d(Tree2D t, double2* __restrict__ b) {
+l2l_leaves2d(Tree2D t, double2* __restrict__ b, const unsigned* err) {
     constexpr int Q = P + 1;
+    if (fatal(err)) return;   // n_leaves is then set, leaf_cells and the cell records need not be
     const int nl = t.info->n_leaves, nc = t.info->n_cells;
     const int dlev = t.dense ? t.dense_levels : 1;
     for (int li = blockIdx.x * blockDim.x + threadIdx.x; li < nl; li += gridDim.x * blockDim.x) {
@@ -159,8 +160,8 @@ cudaError_t launch_m2m_big(const Tree2D& t, Expansions2D& e, int min_count, int 
 }
 
 template <int P>
-cudaError_t launch_l2l_leaves(const Tree2D& t, Expansions2D& e, cudaStream_t st) {
-    l2l_leaves2d<P><<<148 * 8, 32 * kLeafShiftWarps, 0, st>>>(t, e.b);
+cudaError_t launch_l2l_leaves(const Tree2D& t, Expansions2D& e, unsigned* err, cudaStream_t st) {
+    l2l_leaves2d<P><<<148 * 8, 32 * kLeafShiftWarps, 0, st>>>(t, e.b, err);
     return cudaGetLastError();
 }
 
@@ -184,10 +185,9 @@ cudaError_t fmm2d_m2m_big(const Tree2D& t, Expansions2D& e, int P, int min_count
 bool l2l_direct_ok(int P, bool exact) { return P >= 1 && P <= kL2LMaxP && (exact || P <= 17); }
 
 cudaError_t fmm2d_l2l_leaves(const Tree2D& t, Expansions2D& e, int P, unsigned* err, cudaStream_t st, int* launches) {
-    (void)err;
     *launches += 1;
     switch (P) {
-#define VPM_CASE(PP) case PP: return launch_l2l_leaves<PP>(t, e, st);
+#define VPM_CASE(PP) case PP: return launch_l2l_leaves<PP>(t, e, err, st);
         VPM_SHIFT_CASES VPM_CASE(19) VPM_CASE(20) VPM_CASE(21) VPM_CASE(22) VPM_CASE(23) VPM_CASE(24) VPM_CASE(25)
         VPM_CASE(26) VPM_CASE(27) VPM_CASE(28) VPM_CASE(29) VPM_CASE(30)
 #undef VPM_CASE

@@ -583,8 +583,9 @@ m2m3d_one(Tree3D t, int L, unsigned* err) {
     if (L < t.info->depth) m2m3d_level(t, L);
 }
 
-__global__ void count_leaves3d(Tree3D t) {
+__global__ void count_leaves3d(Tree3D t, const unsigned* err) {
     __shared__ int s_red[8];
+    if (block_fatal(err)) return;
     const int nc = t.info->n_cells;
     int k = 0;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) k += t.c_chmask[c] == 0;
@@ -1111,7 +1112,7 @@ cudaError_t build_tree3d(const double* x, const double* y, const double* z, cons
     e = launch_coop(octree_levels3d<false>, kT3Threads, 0, st, 4, &grid, t, x, y, z, act, (uint32_t*)nullptr,
                     kCoopMaxBlocks3D, err);
     if (e != cudaSuccess) return e;
-    count_leaves3d<<<148, 256, 0, st>>>(t);
+    count_leaves3d<<<148, 256, 0, st>>>(t, err);
     *launches += 2;
     return leaves_upward3d(x, y, z, ax, ay, az, act, t, s, err, st, launches);
 }
