@@ -8,12 +8,14 @@
 // first. With use_graph the whole batch - every solve's launches on every
 // stream - is captured once as one CUDA graph and replayed by a single graph
 // launch while the batch layout is unchanged; the first call for a layout
-// tunes S: it captures the batch for each S in kBatchStreamChoices, times two
-// replays of each and keeps the fastest graph (the choice is remembered per
-// layout for the life of the context).
+// tunes S: it captures the batch for each S in kBatchStreamChoices, with a few
+// solves also both ways of capturing a solve (Ctx::branches), times the second
+// of two replays of each and keeps the fastest graph (the choice is remembered
+// per layout for the life of the context).
 #include <algorithm>
 #include <cstring>
 #include <numeric>
+#include <utility>
 
 #include "context.h"
 
@@ -25,6 +27,15 @@ constexpr int kBatchStreamChoices[] = {4, 8, 12, 16};
 constexpr int kBatchStreamsMax = 16;
 constexpr int kBatchStreamsEager = 8;
 constexpr int64_t kSolveFixed = 150000;
+// Solves of a captured batch that fork onto their side streams (up to the
+// first), run in order (from the second on), or are timed both ways: one or two
+// solves leave the GPU to the branches, many fill it without them. Branched
+// against in order: one of 300,000 particles 272 us / 347 (mixed, p = 8, caps
+// 100/150) and 330 / 404 (FP64, p = 10, caps 50/75); two 385 / 456 and 507 / 541;
+// four 641 / 683 and 912 / 871; six 1,021 / 1,114 and 1,420 / 1,409; eight of
+// 60,000 434 / 390 and 663 / 597, of 300,000 1,282 / 1,262 and 1,818 / 1,750.
+constexpr int kBatchBranched = 2;
+constexpr int kBatchInOrder = 8;
 
 // Word 1 of a context's error buffer collects the error bits of every solve
 // the context ran in the current batch (word 0 is reset by each solve).
@@ -66,7 +77,6 @@ int Ctx::prepare_batch(int ns, const int64_t* offs, const vpm_fmm_params& p, int
         // (64 uneven solves: 3.90 ms, against 4.45 with 2048 and 4.08 with 4096; four
         // large ones: 0.56, against 0.64 with 16384)
         c->sort_items = 8192;
-        c->branches = false;
         subs.push_back(c);
         cudaEvent_t e = nullptr;
         VPM_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -121,16 +131,20 @@ int Ctx::enqueue_batch(int ns, const int64_t* offs, const double* x, const doubl
     return VPM_OK;
 }
 
-// One CUDA graph of the whole batch with S streams.
+// One CUDA graph of the whole batch with S streams, each solve forked onto its
+// context's side streams or in order (Ctx::branches).
 int Ctx::capture_batch(int ns, const int64_t* offs, const double* x, const double* y, const double* q,
-                       const uint8_t* act, const vpm_fmm_params& p, double* ex, double* ey, int S,
+                       const uint8_t* act, const vpm_fmm_params& p, double* ex, double* ey, int S, bool branches,
                        cudaGraphExec_t* out) {
     *out = nullptr;
     std::vector<int> stream_of, order;
     plan_batch(ns, offs, S, stream_of, order);
     if (int r = prepare_batch(ns, offs, p, S, stream_of)) return r;
     VPM_CUDA_TRY(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    for (int s = 0; s < S; ++s) subs[s]->capturing = true;
+    for (int s = 0; s < S; ++s) {
+        subs[s]->capturing = true;
+        subs[s]->branches = branches;
+    }
     int r = enqueue_batch(ns, offs, x, y, q, act, p, ex, ey, S, stream_of, order);
     for (int s = 0; s < S; ++s) subs[s]->capturing = false;
     cudaGraph_t g = nullptr;
@@ -186,11 +200,18 @@ int Ctx::batch2d(int ns, const int64_t* offs, const double* x, const double* y, 
     }
     float best_ms = 0.f;
     int best_s = 0;
+    std::vector<std::pair<int, bool>> choices;   // streams, branches
+    const int solves = (int)std::count_if(offs, offs + ns, [&](const int64_t& o) { return (&o)[1] > o; });
     for (int S : kBatchStreamChoices) {
         if (S > std::max(1, ns) && S != kBatchStreamChoices[0]) break;
         const int SS = std::min(S, std::max(1, ns));
+        if (solves > kBatchBranched) choices.push_back({SS, false});
+        if (solves < kBatchInOrder) choices.push_back({SS, true});
+    }
+    for (const auto& choice : choices) {
+        const int SS = choice.first;
         cudaGraphExec_t g = nullptr;
-        if (int r = capture_batch(ns, offs, x, y, q, act, p, ex, ey, SS, &g)) return r;
+        if (int r = capture_batch(ns, offs, x, y, q, act, p, ex, ey, SS, choice.second, &g)) return r;
         float ms = 0.f;
         cudaError_t e = cudaGraphLaunch(g, stream);
         if (e == cudaSuccess) e = cudaEventRecord(tune_ev[0], stream);

@@ -134,12 +134,12 @@ struct Ctx {
     // more in the sub-contexts of a batch, whose solves share the GPU
     int sort_items = 1024;
     // A captured evaluation forks onto the side streams. Off in the
-    // sub-contexts of a batch: the other solves fill the GPU there, and a solve
-    // in order has half the launches, no events and no separate near-field and
-    // spill passes (64 solves of 4,096 to 400,000, mixed: 4.32 -> 3.90 ms; 16 of
-    // 1,000 to 20,000, FP64: 0.655 -> 0.510; 4 of 100,000 to 400,000: 0.571 ->
-    // 0.563; with the branches kept and the one-launch CSR of lists 1/3: 4.02,
-    // 0.543, 0.558).
+    // sub-contexts of a batch of many: the other solves fill the GPU there, and a
+    // solve in order has half the launches, no events and no separate near-field
+    // and spill passes (64 solves of 4,096 to 400,000, mixed: 4.32 -> 3.90 ms; 16
+    // of 1,000 to 20,000, FP64: 0.655 -> 0.510; with the branches kept and the
+    // one-launch CSR of lists 1/3: 4.02, 0.543). batch2d.cu picks, by
+    // kBatchBranched and kBatchInOrder.
     bool branches = true;
 
     // batched solves (batch2d.cu)
@@ -203,7 +203,7 @@ struct Ctx {
                       const uint8_t* act, const vpm_fmm_params& p, double* ex, double* ey, int S,
                       const std::vector<int>& stream_of, const std::vector<int>& order);
     int capture_batch(int ns, const int64_t* offs, const double* x, const double* y, const double* q,
-                      const uint8_t* act, const vpm_fmm_params& p, double* ex, double* ey, int S,
+                      const uint8_t* act, const vpm_fmm_params& p, double* ex, double* ey, int S, bool branches,
                       cudaGraphExec_t* out);
     void drop_batch();
     void drop_graph();
