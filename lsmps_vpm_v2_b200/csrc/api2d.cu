@@ -481,6 +481,9 @@ int Ctx::launch2d(const double* x, const double* y, const double* q, const uint8
     k.n = n; k.K = K; k.velocity = velocity; k.uinf = uinf; k.vinf = vinf; k.p = p; k.stream = stream;
     k.arena = arena2d;
     k.deferred = q_ready != nullptr;
+    // The tables in the arena are those of the last call, which a replay does
+    // not upload; an upload synchronises: never inside a capture.
+    if (int r = ensure_coefs(p)) return r;
     const bool split = p.use_graph == 2;
     const bool have = split ? stage_exec[0] != nullptr : gexec != nullptr;
     if (have && std::memcmp(&k, &gkey, sizeof(k)) == 0) {
@@ -501,7 +504,6 @@ int Ctx::launch2d(const double* x, const double* y, const double* q, const uint8
         return VPM_OK;
     }
     drop_graph();
-    if (int r = ensure_coefs(p)) return r;  // uploads synchronise: never inside a capture
     VPM_CUDA_TRY(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     capturing = true;
     split_capture = split;

@@ -187,6 +187,10 @@ int Ctx::batch2d(int ns, const int64_t* offs, const double* x, const double* y, 
     key.insert(key.end(), pk.begin(), pk.end());
     if (batch_exec && key == batch_key) {
         batch_subs = batch_streams;
+        // an eager batch of another order may have left its tables in the arenas
+        for (int s = 0; s < batch_streams; ++s)
+            if (subs[s]->arena2d)
+                if (int r = subs[s]->ensure_coefs(p)) return fail(r, subs[s]->last_error);
         VPM_CUDA_TRY(cudaGraphLaunch(batch_exec, stream));
         return VPM_OK;
     }
