@@ -113,6 +113,7 @@ int Ctx::reserve2d(int n, int cap_cells, int P, long long cap_l1, long long cap_
     drop_graph();
     if (arena2d) cudaFree(arena2d);
     arena2d = nullptr;
+    ++arena2d_serial;
     cap = Caps2D{};
     cudaError_t e = cudaMalloc(&arena2d, L.total);
     if (e != cudaSuccess) {

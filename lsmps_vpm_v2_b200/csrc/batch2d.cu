@@ -185,7 +185,14 @@ int Ctx::batch2d(int ns, const int64_t* offs, const double* x, const double* y, 
     std::vector<int64_t> pk((sizeof(p) + 7) / 8, 0);
     std::memcpy(pk.data(), &p, sizeof(p));
     key.insert(key.end(), pk.begin(), pk.end());
-    if (batch_exec && key == batch_key) {
+    // the sub-contexts' arenas are part of it: another batch may have had to
+    // lay one out anew, and the graph's launches hold the old addresses
+    auto arenas = [&](int S) {
+        std::vector<unsigned> v;
+        for (int s = 0; s < S; ++s) v.push_back(subs[s]->arena2d_serial);
+        return v;
+    };
+    if (batch_exec && key == batch_key && arenas(batch_streams) == batch_arenas) {
         batch_subs = batch_streams;
         // an eager batch of another order may have left its tables in the arenas
         for (int s = 0; s < batch_streams; ++s)
@@ -212,6 +219,8 @@ int Ctx::batch2d(int ns, const int64_t* offs, const double* x, const double* y, 
         if (solves > kBatchBranched) choices.push_back({SS, false});
         if (solves < kBatchInOrder) choices.push_back({SS, true});
     }
+    // Sub-context s takes the batch's s-th largest solve first whatever the
+    // choice, so no capture enlarges an arena that one before it holds.
     for (const auto& choice : choices) {
         const int SS = choice.first;
         cudaGraphExec_t g = nullptr;
@@ -239,6 +248,7 @@ int Ctx::batch2d(int ns, const int64_t* offs, const double* x, const double* y, 
     batch_subs = best_s;
     batch_streams = best_s;
     batch_key = key;
+    batch_arenas = arenas(best_s);
     VPM_CUDA_TRY(cudaGraphLaunch(batch_exec, stream));
     return VPM_OK;
 }

@@ -72,6 +72,7 @@ struct Ctx {
 
     // 2D arena
     void* arena2d = nullptr;
+    unsigned arena2d_serial = 0;   // counts its layouts (an address may come back with another one)
     size_t arena2d_bytes = 0;
     Caps2D cap;
     bool grow = false;
@@ -148,6 +149,7 @@ struct Ctx {
     cudaEvent_t fork_ev = nullptr;
     cudaGraphExec_t batch_exec = nullptr;
     std::vector<int64_t> batch_key;
+    std::vector<unsigned> batch_arenas;   // arena2d_serial of the sub-contexts the graph runs on
     int batch_subs = 0;
     int batch_streams = 0;                       // streams of the tuned batch graph
     cudaEvent_t tune_ev[2] = {nullptr, nullptr};  // timing of the stream-count tuning
