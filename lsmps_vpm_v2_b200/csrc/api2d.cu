@@ -279,7 +279,7 @@ int Ctx::enqueue2d(const double* x, const double* y, const double* q, const uint
         // to the M2M loop runs on the lists-2/4 stream as soon as the other
         // moments are final, beside that loop; the rest follows it (the FP64
         // M2L split like that: no change, 334 us against 346 at 340k)
-        const bool split = p.precision == VPM_PREC_MIXED && m2l_parent_f32_supported(p.p) &&
+        const bool split = split_m2l && p.precision == VPM_PREC_MIXED && m2l_parent_f32_supported(p.p) &&
                            lists.l2_blk && tree.nonleaf && tree.gbar;
         VPM_CUDA_TRY(fmm2d_upward_direct(tree, ex2, p.p, p.binom == VPM_BINOM_EXACT, d_err, st, &launches,
                                          split ? ev_small : nullptr));

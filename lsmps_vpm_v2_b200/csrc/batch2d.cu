@@ -77,6 +77,7 @@ int Ctx::prepare_batch(int ns, const int64_t* offs, const vpm_fmm_params& p, int
         // (64 uneven solves: 3.90 ms, against 4.45 with 2048 and 4.08 with 4096; four
         // large ones: 0.56, against 0.64 with 16384)
         c->sort_items = 8192;
+        c->split_m2l = false;
         subs.push_back(c);
         cudaEvent_t e = nullptr;
         VPM_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));

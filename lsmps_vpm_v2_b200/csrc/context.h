@@ -142,6 +142,11 @@ struct Ctx {
     // one-launch CSR of lists 1/3: 4.02, 0.543). batch2d.cu picks, by
     // kBatchBranched and kBatchInOrder.
     bool branches = true;
+    // Mixed form, branched: the M2L of the levels below the large cells beside
+    // their M2M loop. Off in the sub-contexts of a batch, whose solves share the
+    // GPU (p = 12, caps 50/75: one of 60,000 particles 203 us without and 216
+    // with it, two 238 and 258, three 282 and 300; one of 300,000 319 and 316).
+    bool split_m2l = true;
 
     // batched solves (batch2d.cu)
     std::vector<Ctx*> subs;
