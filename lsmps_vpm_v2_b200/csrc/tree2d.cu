@@ -282,8 +282,9 @@ static_assert(kCoopSortMaxChunk < 1 << 16, "two counts per word, 16-bit ranks");
 // which the kernel checks after the three passes. Otherwise it sorts again
 // with all four passes.
 //
-// The flat build's per-particle records (pinfo, particle_levels) come with
-// that check: they read the same keys, and a launch of their own took 8 us.
+// The flat build's per-particle records (pinfo, particle_levels; null: not
+// here) come with that check: they read the same keys, and a launch of their
+// own took 8 us.
 //
 // CLUSTER (up to 16 blocks, one thread-block cluster): the same steps with the
 // cluster's hardware barrier (0.3 to 0.6 us, against 1.3 to 2 through a word in
@@ -673,7 +674,7 @@ sort2d_coop(const double* __restrict__ x, const double* __restrict__ y, const do
                 const int j = i + shallow_cap;
                 if (j < n && __ldcg(t.key + i) == __ldcg(t.key + j)) over = true;
             }
-            pinfo[i] = particle_levels(t, i, max_src, max_par);
+            if (pinfo) pinfo[i] = particle_levels(t, i, max_src, max_par);
         }
         if (attempt == 1) break;
         const int any = __syncthreads_or(over);
@@ -1159,6 +1160,7 @@ bool coop_sort_shape(int n, int items, int* grid, int* chunk) {
 // Captured mixed evaluation, cluster against grid: 2,001 particles 98 against
 // 115 us, 20,001 121 against 124, 32,001 127 against 128, 50,001 166 against 155.
 constexpr int kClusterItems = 1024;
+constexpr int kRecordItems = 1024;
 constexpr int kClusterMaxBlocks = 16;
 constexpr int kClusterMaxN = 32768;
 
@@ -1212,6 +1214,11 @@ cudaError_t keys_sort2d(const double* x, const double* y, const double* q, const
         coop_chunk = ceil_div(n, cluster);
     }
     if (cluster || (2 * K <= 32 && s.coop_words && coop_sort_shape(n, items_per_block, &coop_grid, &coop_chunk))) {
+        // Fewer, fuller blocks leave the records' searches to too few threads:
+        // flat_bigl takes them over the whole GPU there (captured batches, 8192
+        // particles a block: one solve of 60,000 197 us, 203 with the records
+        // in the sort, two of 30,000 199 and 205, five of 300,000 1,073 and 1,095).
+        uint32_t* records = items_per_block > kRecordItems ? nullptr : s.pinfo;
         uint32_t* k32 = reinterpret_cast<uint32_t*>(s.key_alt);
         const size_t smem = (size_t)coop_chunk * 10;
         cudaLaunchConfig_t cfg = {};
@@ -1232,9 +1239,9 @@ cudaError_t keys_sort2d(const double* x, const double* y, const double* q, const
         cfg.numAttrs = 1;
         e = cudaLaunchKernelEx(&cfg, cluster ? sort2d_coop<true> : sort2d_coop<false>, x, y, q, act, exp_pct,
                                (2 * K + 7) / 8, shallow_cap, t, s.bbox_partial,
-                               k32, k32 + n, s.val_alt, t.perm, s.coop_words, coop_chunk, max_src, max_par, s.pinfo,
+                               k32, k32 + n, s.val_alt, t.perm, s.coop_words, coop_chunk, max_src, max_par, records,
                                err);
-        s.pinfo_done = true;
+        s.pinfo_done = records != nullptr;
         if (e != cudaSuccess) return e;
         *launches += 1;
         return cudaGetLastError();
