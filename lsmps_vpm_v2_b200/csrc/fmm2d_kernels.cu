@@ -697,7 +697,8 @@ __device__ __forceinline__ double log_series(double a) {
 }
 
 // Staged sources s0, s0 + ns, ... below cnt onto the lane's M targets; SELF:
-// flat source self[k] is target k itself. POT: sums q log(r^2) in ex.
+// flat source self[k] is target k itself and adds zero whatever its strength.
+// POT: sums q log(r^2) in ex.
 template <int M, bool POT, bool SELF>
 __device__ __forceinline__ void near64_pairs(const double2* xy, const double* q, int s0, int cnt, int ns,
                                              const double* x, const double* y, const int* self, double* ex,
@@ -735,7 +736,7 @@ __device__ __forceinline__ void near64_pairs(const double2* xy, const double* q,
                     if (!log_ordinary(r2[k])) lg[k] = SELF && s == self[k] ? 0.0 : log(r2[k]);
             }
             #pragma unroll
-            for (int k = 0; k < M; ++k) ex[k] = fma(w, lg[k], ex[k]);
+            for (int k = 0; k < M; ++k) ex[k] = fma(SELF && s == self[k] ? 0.0 : w, lg[k], ex[k]);
         }
     }
 }
