@@ -884,11 +884,15 @@ near2d_f64(Tree2D t, Lists2D l, const double* __restrict__ fx, const double* __r
     const int nl = t.info->n_leaves;
     // A tree of few leaves leaves most of the GPU's 148 x 12 warps without one:
     // 2, 4 or 8 warps then share a leaf's targets (2,001 particles, 64 leaves:
-    // 24 -> 12 us). Splitting further than one warp per place costs more in
-    // repeated staging than it evens out (20,001 particles, about 1,024 leaves
-    // in 2 and 4 parts: the graph 133 -> 144 and 156 us).
+    // 24 -> 12 us), up to half the GPU's places. Each part stages the leaf's
+    // sources again, which costs other solves the GPU when they share it: with
+    // all places taken, 256 leaves in four parts in place of two, a captured batch
+    // of 24 solves of 6,000 particles took 782 us (735 with this line, 711 with a
+    // quarter of the places, 706 without parts), one of 48 1,408 (1,316, 1,263,
+    // 1,250); alone, 12,000 particles of as many leaves 169, 170, 174 and 174 us
+    // eager. 20,001 particles, about 1,024 leaves: 133 us in one part, 144 in two.
     int parts = 1;
-    while (parts < 8 && (long long)nl * parts * 2 <= 148 * 12) parts *= 2;
+    while (parts < 8 && (long long)nl * parts * 2 <= 148 * 6) parts *= 2;
     for (int it = blockIdx.x * kNear64Warps + wib; it < nl * parts; it += gridDim.x * kNear64Warps) {
         const int li = it / parts, part = it - li * parts;
         const int32_t* src1;
