@@ -671,7 +671,7 @@ sort2d_coop(const double* __restrict__ x, const double* __restrict__ y, const do
         bool over = false;
         for (int i = c0 + tid; i < c1; i += kCoopSortThreads) {
             if (attempt == 0) {
-                const int j = i + shallow_cap;
+                const long long j = (long long)i + shallow_cap;
                 if (j < n && __ldcg(t.key + i) == __ldcg(t.key + j)) over = true;
             }
             if (pinfo) pinfo[i] = particle_levels(t, i, max_src, max_par);
