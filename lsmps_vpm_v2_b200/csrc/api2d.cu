@@ -372,12 +372,18 @@ int Ctx::enqueue2d(const double* x, const double* y, const double* q, const uint
 
 // Whether the FP64 M2L goes per parent cell: its blocks take 32 parents at
 // once, so a small tree leaves most of the GPU idle and is faster with a warp
-// per target cell. The line is drawn by the expected number of leaves: at cap
-// 50, 50,001 scattered particles 153 us with a warp per cell and 160 per
-// parent (captured graph), a 65,536-particle lattice 172 and 166, 120,001
-// particles 185 and 178, 340,000 particles 400 and 335.
+// per target cell. The line is drawn by the expected number of leaves and is
+// the same for an eager and a captured call, whose results are the same bits.
+// A warp per cell against per parent, caps 50/75: captured, p = 10, 40,000
+// scattered particles 129 us and 138, 60,000 165 and 155, 200,000 248 and 230;
+// in order, where nothing runs beside it, the sides meet later (p = 10, 90,000:
+// 232 and 235, 200,000: 350 and 349, 300,000: 431 and 407). Above p = 14 the
+// kernel's registers spill and one block fills an SM's shared memory: captured,
+// p = 16, 60,000 187 and 195, 130,000 204 and 218, 200,000 288 and 281, 300,000
+// 427 and 375; in order 200,000 399 and 404, 300,000 559 and 506.
 bool Ctx::m2l_f64_per_parent(const vpm_fmm_params& p) const {
-    return m2l_parent_f64_supported(tree, lists, p.p) && tree.n / std::max(1, std::min(p.max_src, p.max_par)) >= 1200;
+    const int leaves = p.p <= 14 ? 1200 : 4000;
+    return m2l_parent_f64_supported(tree, lists, p.p) && tree.n / std::max(1, std::min(p.max_src, p.max_par)) >= leaves;
 }
 
 // M2L of lists 2 and 4 for the precision setting: the mixed form per parent
