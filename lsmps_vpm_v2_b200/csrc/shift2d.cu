@@ -90,11 +90,15 @@ m2m_big_levels_coop(Tree2D t, double2* __restrict__ a, int min_count, const unsi
 // rounding (shifts of a degree-P polynomial compose exactly), without a level
 // loop or a grid barrier. Ancestors come from the dense grid (written for
 // every cell of levels <= dense_levels by the tree build, so an ancestor's
-// entry is always current) and, below it, the parent chain. The next
-// ancestor's index and centre are loaded while the current part is shifted.
+// entry is always current) and, below it, the parent chain, walked once. The
+// next ancestor's index and centre are loaded while the current part is shifted.
 // 778,377-particle boundary layer, P = 10: 14 us (37 with a lane per
 // coefficient, P + 1 of 32 lanes on a leaf); 530,888 particles, P = 16: 20 us
-// (80).
+// (80). Above P = 16 the registers of two expansions grow, and from 27 on they
+// spill: 600,000 particles, P = 17, 20, 24, 27, 30: 18, 23, 29, 35, 41 us (57, 57,
+// 72, 72, 76); 100,000: 12, 14, 16, 18, 23 (18, 18, 21, 23, 23). Leaves down to
+// level 27 (6,000 particles in eight nested blobs), P = 16: 37 us (38, and 41
+// with a walk of the chain for every level).
 constexpr int kLeafShiftWarps = 2;   // few leaves per SM: small blocks spread them
 
 template <int P>
@@ -109,15 +113,11 @@ l2l_leaves2d(Tree2D t, double2* __restrict__ b, const unsigned* err) {
         const int L = t.c_level[c];
         if (L <= 2) continue;
         const int ix = t.c_ix[c], iy = t.c_iy[c];
+        int chain[kMaxLevels2D];   // ancestors below the dense grid, from one walk up
+        for (int l = L - 1, a = c; l > dlev && l >= 2; --l) chain[l] = a = t.c_parent[a];
         auto ancestor = [&](int m) {
             const int sh = L - m;
-            int a = -1;
-            if (m <= dlev) {
-                a = t.dense[start_id2(m) + (ix >> sh) + ((int64_t)(iy >> sh) << m)];
-            } else {
-                a = c;
-                for (int l = L; l > m; --l) a = t.c_parent[a];
-            }
+            const int a = m <= dlev ? t.dense[start_id2(m) + (ix >> sh) + ((int64_t)(iy >> sh) << m)] : chain[m];
             return a >= 0 && a < nc ? a : c;   // always a cell; c itself would add nothing wrong to read
         };
         auto centre = [&](int a) { return make_double2(t.c_cx[a], t.c_cy[a]); };
