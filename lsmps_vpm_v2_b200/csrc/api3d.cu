@@ -60,7 +60,7 @@ int Ctx::reserve3d(int n, int cap_cells) {
     size_t o_np = L.take<int32_t>(C), o_par = L.take<int32_t>(C), o_ch0 = L.take<int32_t>(C),
            o_lo = L.take<int32_t>(C), o_hi = L.take<int32_t>(C);
     size_t o_mask = L.take<uint32_t>(C), o_act2 = L.take<uint8_t>(C), o_lev = L.take<uint8_t>(C);
-    size_t o_mom = L.take<double>(C * kMom3D), o_leaves = L.take<int32_t>(C);
+    size_t o_mom = L.take<double>(C * kMom3D);
     size_t o_ps32 = L.take<float4>(n), o_as32 = L.take<float4>(n), o_rec32 = L.take<float>(C * kRec32Floats);
     size_t o_gbar = L.take<unsigned>(8), o_blk = L.take<uint32_t>(kCoopMaxBlocks3D);
     size_t o_geom = L.take<Geom3D>(1), o_info = L.take<TreeInfo3D>(1), o_bbox = L.take<double>(296 * 6);
@@ -98,7 +98,7 @@ int Ctx::reserve3d(int n, int cap_cells) {
     t.c_npar = (int32_t*)P_(o_np); t.c_parent = (int32_t*)P_(o_par); t.c_child0 = (int32_t*)P_(o_ch0);
     t.c_lo = (int32_t*)P_(o_lo); t.c_hi = (int32_t*)P_(o_hi);
     t.c_chmask = (uint32_t*)P_(o_mask); t.c_active = (uint8_t*)P_(o_act2); t.c_level = (uint8_t*)P_(o_lev);
-    t.mom = (double*)P_(o_mom); t.leaf_cells = (int32_t*)P_(o_leaves);
+    t.mom = (double*)P_(o_mom);
     t.ps32 = (float4*)P_(o_ps32); t.as32 = (float4*)P_(o_as32); t.rec32 = (float*)P_(o_rec32);
     t.gbar = (unsigned*)P_(o_gbar); t.blk = (uint32_t*)P_(o_blk);
     t.geom = (Geom3D*)P_(o_geom); t.info = (TreeInfo3D*)P_(o_info);

@@ -24,7 +24,6 @@ namespace vpm {
 namespace {
 
 constexpr int kBatchStreamChoices[] = {4, 8, 12, 16};
-constexpr int kBatchStreamsMax = 16;
 constexpr int kBatchStreamsEager = 8;
 constexpr int64_t kSolveFixed = 150000;
 // Solves of a captured batch that fork onto their side streams (up to the

@@ -644,7 +644,6 @@ struct Near64Warp {
         double red[2 * kNear64MaxM][32];
     };
     int2 meta[kP2PMeta];       // first particle and size of each list-1 cell
-    int cs[kP2PMeta + 1];      // its flat start, then the total
 };
 
 // Targets per lane of a chunk of T: the least (10 M + 3) / ns, ten operations
@@ -787,8 +786,6 @@ __device__ __forceinline__ void near64_chunk(Near64Warp& sm, const Tree2D& t, co
         const int tot0 = __shfl_sync(0xffffffffu, inc[0], 31);
         const int total = tot0 + __shfl_sync(0xffffffffu, inc[1], 31);
         const int start0 = inc[0] - sz[0], start1 = tot0 + inc[1] - sz[1];
-        if (lane < nseg) sm.cs[lane] = start0;
-        if (lane + 32 < nseg) sm.cs[lane + 32] = start1;
         const unsigned b0 = __ballot_sync(0xffffffffu, own[0]), b1 = __ballot_sync(0xffffffffu, own[1]);
         int own0 = -(1 << 30);
         if (b0) own0 = __shfl_sync(0xffffffffu, start0, __ffs(b0) - 1);

@@ -74,7 +74,6 @@ struct Tree3D {
     float4* ps32;                     // position minus its leaf's centre, active flag in .w
     float4* as32;                     // alpha
     float* rec32;                     // [cap_cells][kRec32Floats]: centre (doubles), moments
-    int32_t* leaf_cells;              // leaves in cell order
     unsigned* gbar;                   // grid barrier words, the octree's kDeepWord; zeroed per evaluation
     uint32_t* blk;                    // per-block scan partials [gridDim]
 };

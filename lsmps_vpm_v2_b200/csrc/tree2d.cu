@@ -966,7 +966,7 @@ flat_scan(Tree2D t, uint32_t* __restrict__ tile_cnt, int tiles, uint32_t* __rest
 // the block at its barrier.
 __global__ void __launch_bounds__(kFlatTile, 8)
 flat_emit(Tree2D t, const uint32_t* __restrict__ pinfo, const uint32_t* __restrict__ tile_cnt, int tiles,
-          int max_par, unsigned* err) {
+          unsigned* err) {
     constexpr int NW = kFlatTile / 32;
     __shared__ unsigned s_mc[kMaxLevels2D + 1][NW], s_ml[kMaxLevels2D + 1][NW];   // lanes with a cell / leaf at L
     __shared__ int s_c0[kMaxLevels2D + 1], s_l0[kMaxLevels2D + 1];   // the tile's first cell / leaf of each level
@@ -1080,7 +1080,7 @@ flat_emit(Tree2D t, const uint32_t* __restrict__ pinfo, const uint32_t* __restri
 // ends where the next sibling of its nearest ancestor-or-self that has one
 // starts (a walk up the parent links, one level per step; most cells stop at
 // their own next sibling), or at n.
-__global__ void flat_link(Tree2D t, int max_par, unsigned* err) {
+__global__ void flat_link(Tree2D t, unsigned* err) {
     if (fatal(err)) return;
     const int nc = t.info->n_cells, n = t.n;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x + 1; c < nc; c += gridDim.x * blockDim.x) {
@@ -1309,9 +1309,9 @@ cudaError_t levels2d_flat(Tree2D& t, TreeScratch2D& s, int max_src, int max_par,
     flat_cells<<<grid, kFlatTile, 0, st>>>(t, s.pinfo, s.tile_cnt, tiles, err);
     // lvl_ticket[0]: zeroed with the other tickets before the sort
     flat_scan<<<2 * (t.key_levels + 1), 1024, 0, st>>>(t, s.tile_cnt, tiles, s.level_tot, s.lvl_ticket, err);
-    flat_emit<<<grid, kFlatTile, 0, st>>>(t, s.pinfo, s.tile_cnt, tiles, max_par, err);
+    flat_emit<<<grid, kFlatTile, 0, st>>>(t, s.pinfo, s.tile_cnt, tiles, err);
     const int gc = std::max(1, std::min(148 * 8, ceil_div(t.cap_cells, 256)));
-    flat_link<<<gc, 256, 0, st>>>(t, max_par, err);
+    flat_link<<<gc, 256, 0, st>>>(t, err);
     *launches += 4;
     return cudaGetLastError();
 }
