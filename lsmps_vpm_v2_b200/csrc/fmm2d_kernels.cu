@@ -8,22 +8,24 @@
 //   fmm2d_upward_direct  moments of every cell of at most 1024 particles
 //                 straight from its particles (upward_direct2d), then M2M of
 //                 the larger cells level by level in one cooperative launch
-//                 (m2m_big_levels_coop), with an optional event between the
-//                 two; fmm2D.cpp:237-284, 309-379.
+//                 (m2m_big_levels_coop, shift2d.cu), with an optional event
+//                 between the two; fmm2D.cpp:237-284, 309-379.
 //   fmm2d_upward  P2M of every active leaf, then M2M over all levels (p2m2d,
 //                 m2m_levels_coop), for orders the direct form does not cover.
 //   fmm2d_m2l_only  lists 2 and 4 of every cell at level >= 2 in FP64 with the
-//                 49 precomputed list-2 operators (m2l2d_op, fmm2D.cpp:396-556);
-//                 the mixed forms' per-parent list-2 M2L is in m2l_tc.cu.
-//   fmm2d_l2l_leaves, fmm2d_l2l  every leaf's local expansion from its
-//                 ancestors' M2L parts, or the level loop (fmm2D.cpp:587-651).
+//                 49 precomputed list-2 operators (m2l2d_op, fmm2D.cpp:396-556),
+//                 in small trees and at high orders; the list-2 M2L per parent
+//                 is in m2l_f64.cu (plain form) and m2l_tc.cu (mixed forms).
+//   fmm2d_l2l     the L2L level loop (fmm2D.cpp:587-651), where the leaves' local
+//                 expansions straight from their ancestors' M2L parts
+//                 (fmm2d_l2l_leaves, shift2d.cu) do not apply.
 //   fmm2d_eval, fmm2d_m2p, fmm2d_eval_combine  M2P over list 3
 //                 (fmm2D.cpp:1040-1066) and L2P (fmm2D.cpp:1076-1093), warp per
 //                 leaf; the combine pass adds the near field and writes the
 //                 output in the caller's order.
 //   fmm2d_p2p_f64, fmm2d_p2p_f32, fmm2d_p2p_potential  near field over list 1, j != i
-//                 (fmm2D.cpp:135-179): FP64 warp kernel for the plain form,
-//                 packed FP32 tiles for the mixed forms.
+//                 (fmm2D.cpp:135-179): FP64 (near2d_f64) for the plain form
+//                 and the potential, packed FP32 tiles for the mixed forms.
 #include "fmm2d.cuh"
 
 #include <complex>

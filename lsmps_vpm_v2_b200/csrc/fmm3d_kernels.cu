@@ -729,10 +729,12 @@ cudaError_t eval3d(const Tree3D& t, bool mixed, bool all_src, const uint8_t* tar
                    double* v, double* w, double uinf, double vinf, double winf, unsigned* err, cudaStream_t st,
                    int* launches) {
     // Warps per block: with at most two blocks per SM the work of one block is
-    // the kernel's time, so eight warps share it (5,202 particles, 82 blocks:
-    // 0.30 ms per call against 0.33 with four); with more blocks than that
-    // four, whose barriers and uneven shares cost less (27,872 particles, 436
-    // blocks: 0.57 against 0.58; 222,688 particles: 3.17 against 3.58).
+    // the kernel's time, so eight warps share it; with more blocks than that
+    // four, whose barriers and uneven shares cost less. A whole call with eight
+    // warps against four, FP64 (mixed): 5,202 particles 228 us against 254 (244,
+    // 288), 14,200 313 and 326 (346, 354), 19,500, where the line lies, 375 and 377
+    // (418, 413), 27,872 424 and 410 (490, 434), 222,688 2,574 and 2,161 (3,239,
+    // 2,238).
     const bool wide = ceil_div(t.n, 64) <= 2 * 148;
 #define VPM_LAUNCH(F, A)                                                                              \
     (wide ? launch_eval3d_w<F, A, 8>(t, target, support, u, v, w, uinf, vinf, winf, err, st)          \

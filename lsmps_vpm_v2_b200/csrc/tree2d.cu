@@ -1154,13 +1154,16 @@ bool coop_sort_shape(int n, int items, int* grid, int* chunk) {
 
 // Blocks of the cluster sort for n particles, about kClusterItems each, or 0
 // when the grid version takes the call: more particles than 16 blocks sort in
-// less time than the grid's SMs, a solve that shares the GPU (items_per_block
-// above 1024: its sorts already overlap others' work), or a device that cannot
-// place the cluster.
+// less time than the grid's SMs, a solve of a batch (items_per_block above
+// 1024), or a device that cannot place the cluster.
 // Captured mixed evaluation, cluster against grid: 2,001 particles 98 against
 // 115 us, 20,001 121 against 124, 32,001 127 against 128, 50,001 166 against 155.
+// In a batch a cluster waits for up to 16 SMs that are free at once: solves of
+// 8,000 particles gain by it (16 of them, FP64: 557 -> 492 us), uneven ones lose
+// (20 of 2,000 to 300,000 particles, FP64 1,610 -> 1,658 us, mixed 1,173 -> 1,231;
+// 64 of them 3,849 -> 3,903 and 2,684 -> 2,798).
 constexpr int kClusterItems = 1024;
-constexpr int kRecordItems = 1024;
+constexpr int kRecordItems = 1024;   // see keys_sort2d
 constexpr int kClusterMaxBlocks = 16;
 constexpr int kClusterMaxN = 32768;
 
