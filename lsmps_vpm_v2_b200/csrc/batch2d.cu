@@ -192,10 +192,12 @@ int Ctx::batch2d(int ns, const int64_t* offs, const double* x, const double* y, 
         for (int s = 0; s < S; ++s) v.push_back(subs[s]->arena2d_serial);
         return v;
     };
-    if (batch_exec && key == batch_key && arenas(batch_streams) == batch_arenas) {
-        batch_subs = batch_streams;
+    const int S0 = (int)batch_arenas.size();   // the graph's; an eager batch since may have run on fewer
+    if (batch_exec && key == batch_key && arenas(S0) == batch_arenas) {
+        batch_subs = S0;
+        batch_streams = S0;
         // an eager batch of another order may have left its tables in the arenas
-        for (int s = 0; s < batch_streams; ++s)
+        for (int s = 0; s < S0; ++s)
             if (subs[s]->arena2d)
                 if (int r = subs[s]->ensure_coefs(p)) return fail(r, subs[s]->last_error);
         VPM_CUDA_TRY(cudaGraphLaunch(batch_exec, stream));
