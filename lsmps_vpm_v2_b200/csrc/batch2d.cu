@@ -103,6 +103,8 @@ int Ctx::enqueue_batch(int ns, const int64_t* offs, const double* x, const doubl
                        const uint8_t* act, const vpm_fmm_params& p, double* ex, double* ey, int S,
                        const std::vector<int>& stream_of, const std::vector<int>& order) {
     cudaError_t e = cudaEventRecord(fork_ev, stream);
+    // the context's own error word may still hold what its last call reported
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_err, 0, sizeof(unsigned), stream);
     for (int s = 0; s < S && e == cudaSuccess; ++s) {
         e = cudaStreamWaitEvent(subs[s]->stream, fork_ev, 0);
         if (e == cudaSuccess) e = cudaMemsetAsync(subs[s]->d_err + 1, 0, sizeof(unsigned), subs[s]->stream);
@@ -355,6 +357,7 @@ int vpm_fmm2d_field_batched(vpm_ctx* ctx, int32_t n_solves, const int64_t* offse
         if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return c->fail_cuda(e, "batched solves");
         unsigned bits = 0;
         if ((r = c->batch_errors(&bits))) return r;
+        c->batch_subs = 0;   // reported here: not by a later vpm_ctx_sync
         if ((bits & vpm::ERR_DEPTH) && p.max_depth < vpm::kMaxLevels2D) {
             p.max_depth = vpm::kMaxLevels2D;  // coincident clusters: resolve 31 levels
             continue;
