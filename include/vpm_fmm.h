@@ -277,7 +277,8 @@ int vpm_batch_streams(vpm_ctx* ctx, int32_t* streams);
  *   fmm3D::get_Field_x / _y / _z                              src/FMM/fmm3D.hpp:106-138
  * Every particle is a target, as in the reference (which ignores the target
  * flags); `target` may be NULL. precision = VPM_PREC_MIXED evaluates the P2P
- * and M2P terms in FP32 (FP64 geometry, decisions and per-target sums).
+ * and M2P terms in FP32 (FP64 geometry, decisions and per-target sums); it is not
+ * the faster form in 3D (2,009,183 particles: 21.9 ms, VPM_PREC_FP64 21.2).
  * Leaf iff particle count < prm->leaf_cap_3d; the root box is the particle
  * box joined with prm->center_3d. Host buffers; stats may be NULL.
  */

@@ -667,7 +667,7 @@ __device__ __forceinline__ int near_shape(int T) {
 }
 
 // log a in FP64 without branches, so that the lane's targets run side by side
-// (CUDA's own log branches for its special cases: 94 us against 53 for the
+// (CUDA's own log branches for its special cases: 94 us against 55 for the
 // near field of 120,011 particles): a = m 2^e with m in [sqrt(1/2), sqrt(2)),
 // log m = 2 atanh z, z = (m - 1) / (m + 1), by the series of atanh to z^21
 // (|z| <= 0.172: the next term is below 2^-60 of the sum; relative error at
