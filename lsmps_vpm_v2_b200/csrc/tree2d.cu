@@ -1135,7 +1135,8 @@ bool coop_sort_shape(int n, int items, int* grid, int* chunk) {
     const int g = std::max(std::max(1, ceil_div(n, kCoopSortMaxChunk)),
                            std::min(std::min(sms, kCoopSortGridMax), ceil_div(n, items)));
     const int c = ceil_div(n, g);
-    if (c > kCoopSortMaxChunk) return false;
+    // more blocks than SMs (above 148 x 16,384 particles) cannot all be resident
+    if (c > kCoopSortMaxChunk || g > std::min(sms, kCoopSortGridMax)) return false;
     if (smem_set == 0) {
         if (cudaFuncSetAttribute(sort2d_coop<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  kCoopSortMaxChunk * 10) != cudaSuccess)
