@@ -67,7 +67,8 @@ int Ctx::prepare_batch(int ns, const int64_t* offs, const vpm_fmm_params& p, int
     while ((int)subs.size() < S) {
         Ctx* c = new (std::nothrow) Ctx();
         if (!c) return fail(VPM_ENOMEM, "sub-context");
-        if (int r = c->init(device)) {
+        // never blocking: it is captured, and then no thread could use the legacy stream
+        if (int r = c->init(device, cudaStreamNonBlocking)) {
             std::string m = c->last_error;
             delete c;
             return fail(r, "sub-context: " + m);

@@ -72,13 +72,13 @@ Ctx::~Ctx() {
         if (x) cudaEventDestroy(x);
 }
 
-int Ctx::init(int dev) {
+int Ctx::init(int dev, unsigned stream_flags) {
     device = dev;
     cudaError_t e = cudaSetDevice(dev);
     if (e != cudaSuccess) return fail_cuda(e, "cudaSetDevice");
-    // A blocking stream: work the caller puts on the legacy default stream
-    // (e.g. PyTorch's default) is ordered with the context's work.
-    e = cudaStreamCreate(&own_stream);
+    // By default a blocking stream: work the caller puts on the legacy default
+    // stream (e.g. PyTorch's default) is ordered with the context's work.
+    e = cudaStreamCreateWithFlags(&own_stream, stream_flags);
     if (e != cudaSuccess) return fail_cuda(e, "cudaStreamCreate");
     stream = own_stream;
     e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);

@@ -170,7 +170,8 @@ struct Ctx {
     HostTree2D host_tree;
 
     ~Ctx();
-    int init(int dev);
+    // stream_flags: of the context's own stream, blocking by default
+    int init(int dev, unsigned stream_flags = cudaStreamDefault);
     int fail(int status, const std::string& msg);
     int fail_cuda(cudaError_t e, const char* what);
     int map_err(unsigned bits);
